@@ -128,13 +128,17 @@ struct TransportArgs {
 // functions on the IBM RISC System/6000 processor", IBM J. Res. Dev. 34(1),
 // 1990): q = RN(num rdx) is within one ulp of num/dx, the remainder
 // r = num - dx q is exact in one fma, and RN(q + r rdx) is the correctly
-// rounded quotient.  A zero numerator is returned as is (keeps its sign).
+// rounded quotient.  The remainder is formed with the opposite sign, dx q - num,
+// so that a zero numerator keeps its sign without a test of its own: for
+// num = -0 it is (-0) + (+0) = +0 and the last step (-0) + (-0) = -0.  Three
+// instructions; with the test they were five, six divisions to a node of the
+// transport and to a node and level of the vertical velocity, whose time is
+// their instruction count.
 template <typename T>
 __device__ __forceinline__ T div_dx(T num, T dx, T rdx) {
   const T q = num * rdx;
-  const T r = fma(-q, dx, num);
-  const T d = fma(r, rdx, q);
-  return num == T(0) ? num : d;
+  const T t = fma(q, dx, -num);
+  return fma(-t, rdx, q);
 }
 
 template <typename T>
@@ -444,8 +448,10 @@ template <typename T>
 struct VertFlowArgs {
   int nz, ny, nx;
   T dx, rdx;               // rdx = RN(1/dx) in T
-  T lev[IGM_MAX_NZ];       // levels (zeta map of compute_levels)
+  T ddz[IGM_MAX_NZ];       // level k minus level k - 1 (zeta map of compute_levels), 0 for k = 0
   T w[IGM_MAX_NZ];         // vert_weight
+  T sw[IGM_MAX_NZ];        // running sum of the weights, in T
+  T rsw[IGM_MAX_NZ];       // RN(1/sw)
   const T* U;
   const T* V;
   const T* topg;
@@ -472,83 +478,118 @@ __device__ __forceinline__ double ieee_div<double>(double a, double b) { return 
 // is built with -fmad=false; every quotient is the correctly rounded one, by
 // Markstein's step from the divisor's correctly rounded reciprocal -- dx, and
 // per layer the sum of the weights), so W is bit-identical.
-constexpr int kVfRows = 8;   // output rows per warp
+//
+// What bounds it is the instruction count (72 % of the issue slots used at
+// 1500 x 1500 x 10).  So each face between two nodes is evaluated once -- in x
+// by the lane on its right, which hands it to the lane on its left, in y by the
+// thread for its two rows (the halves are exact and the sums commute, so both
+// nodes see the same bits) -- and strips and segments that touch no border of
+// the domain (EDGE false: all but the outermost) carry no border formulas.
+// 1000 x 1000 x 10 FP32: 57.0 -> 45.1 us (2.25 -> 2.84 TB/s).  Rows per warp and
+// CTAs per SM, measured there: 8 rows at 4 CTAs 48.9, at 3 49.4, at 5 (spilling)
+// 60.0; 6 rows at 5 45.1, at 6 52.9; 4 rows at 6 47.7, at 8 51.5.
+constexpr int kVfRows = 6;   // output rows per warp
 constexpr int kVfCols = 30;  // output columns per warp
 constexpr int kVfWarps = 4;  // warps per CTA
-template <typename T>
-__global__ void __launch_bounds__(kVfWarps * 32) vert_flow_kernel(const VertFlowArgs<T> a, int n_strips) {
+template <typename T, bool EDGE>
+__device__ __forceinline__ void vert_flow_march(const VertFlowArgs<T>& a, int lane, int strip, int j0) {
   constexpr int R = kVfRows + 2;
-  const int lane = threadIdx.x & 31;
-  const int gw = blockIdx.x * kVfWarps + (threadIdx.x >> 5);
-  const int strip = gw % n_strips, seg = gw / n_strips;
   const int nx = a.nx, ny = a.ny;
-  const int j0 = seg * kVfRows;
-  if (j0 >= ny) return;  // uniform per warp
   const int i = strip * kVfCols - 1 + lane;
-  const bool col = i >= 0 && i < nx;
-  const size_t ic = col ? (size_t)i : 0;
+  const bool col = !EDGE || (i >= 0 && i < nx);
   const size_t plane = (size_t)ny * nx;
   const bool out_lane = lane >= 1 && lane <= kVfCols && col;
-  const T dx = a.dx, rdx = a.rdx;
+  const T dx = a.dx, rdx = a.rdx, h = T(0.5), o5 = T(1.5);
+  const size_t o0 = EDGE ? (col ? (size_t)i : 0) : (size_t)(j0 - 1) * nx + i;  // EDGE: the column, else the first node
+  auto at = [&](const T* p, int r) -> T {
+    if (!EDGE) return p[o0 + (size_t)r * nx];
+    const int j = j0 - 1 + r;
+    return (col && j >= 0 && j < ny) ? p[(size_t)j * nx + o0] : T(0);
+  };
   T tg[R], th[R], zh[R], su[R], sv[R];
-  bool in[R];
-  size_t off[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    const int j = j0 - 1 + r;
-    in[r] = col && j >= 0 && j < ny;
-    off[r] = in[r] ? (size_t)j * nx + ic : 0;
-    tg[r] = in[r] ? a.topg[off[r]] : T(0);
-    th[r] = in[r] ? a.thk[off[r]] : T(0);
+    tg[r] = at(a.topg, r);
+    th[r] = at(a.thk, r);
     zh[r] = T(0);
     su[r] = T(0);
     sv[r] = T(0);
   }
-  T sw = T(0);
-  for (int k = 0; k < a.nz; ++k) {
+  const T *U = a.U, *V = a.V;
+  T* W = a.W;
+  for (int k = 0; k < a.nz; ++k, U += plane, V += plane, W += plane) {
     T u[R], v[R], z[R], qx[R], qy[R];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-      u[r] = in[r] ? a.U[(size_t)k * plane + off[r]] : T(0);
-      v[r] = in[r] ? a.V[(size_t)k * plane + off[r]] : T(0);
+      u[r] = at(U, r);
+      v[r] = at(V, r);
     }
-    sw = k == 0 ? a.w[0] : sw + a.w[k];
-    const T rsw = ieee_div(T(1), sw);  // the layer's one divisor: Markstein's step from its reciprocal
-    const T ddz = k > 0 ? a.lev[k] - a.lev[k - 1] : T(0);
+    const T sw = a.sw[k], rsw = a.rsw[k];  // the layer's one divisor: Markstein's step from its reciprocal
+    const T ddz = a.ddz[k], wk = a.w[k];
 #pragma unroll
     for (int r = 0; r < R; ++r) {
       if (k > 0) {
         const T dzl = th[r] * ddz;
         zh[r] = k == 1 ? dzl : zh[r] + dzl;
       }
-      const T wu = a.w[k] * u[r], wv = a.w[k] * v[r];
+      const T wu = wk * u[r], wv = wk * v[r];
       su[r] = k == 0 ? wu : su[r] + wu;
       sv[r] = k == 0 ? wv : sv[r] + wv;
       z[r] = tg[r] + zh[r];
       qx[r] = div_dx(su[r], sw, rsw) * zh[r];
       qy[r] = div_dx(sv[r], sw, rsw) * zh[r];
     }
+    // the faces below row 1: of the layer surface (compute_gradient_layers_tf) and of the fluxes
+    // (compute_divflux_layers)
+    T zs = h * z[0] + h * z[1], fs = h * (qy[0] + qy[1]);
+    if (EDGE && j0 == 0) {
+      zs = o5 * z[1] - h * z[2];
+      fs = qy[1];
+    }
 #pragma unroll
     for (int r = 1; r <= kVfRows; ++r) {
       const int j = j0 - 1 + r;
-      const T zl = __shfl_up_sync(0xffffffffu, z[r], 1), zr = __shfl_down_sync(0xffffffffu, z[r], 1);
-      const T ql = __shfl_up_sync(0xffffffffu, qx[r], 1), qr = __shfl_down_sync(0xffffffffu, qx[r], 1);
-      if (!out_lane || j >= ny) continue;
-      // faces of the layer surface (compute_gradient_layers_tf)
-      const T zw = i == 0 ? T(1.5) * z[r] - T(0.5) * zr : T(0.5) * zl + T(0.5) * z[r];
-      const T ze = i == nx - 1 ? T(1.5) * z[r] - T(0.5) * zl : T(0.5) * z[r] + T(0.5) * zr;
-      const T zs = j == 0 ? T(1.5) * z[r] - T(0.5) * z[r + 1] : T(0.5) * z[r - 1] + T(0.5) * z[r];
-      const T zn = j == ny - 1 ? T(1.5) * z[r] - T(0.5) * z[r - 1] : T(0.5) * z[r] + T(0.5) * z[r + 1];
-      // faces of the fluxes (compute_divflux_layers)
-      const T fw = i == 0 ? qx[r] : T(0.5) * (ql + qx[r]);
-      const T fe = i == nx - 1 ? qx[r] : T(0.5) * (qx[r] + qr);
-      const T fs = j == 0 ? qy[r] : T(0.5) * (qy[r - 1] + qy[r]);
-      const T fn = j == ny - 1 ? qy[r] : T(0.5) * (qy[r] + qy[r + 1]);
+      // this lane's left faces; the right ones are the left ones of the lane beside it
+      const T zl = __shfl_up_sync(0xffffffffu, z[r], 1), ql = __shfl_up_sync(0xffffffffu, qx[r], 1);
+      T zw = h * zl + h * z[r], fw = h * (ql + qx[r]);
+      if (EDGE) {
+        const T zr = __shfl_down_sync(0xffffffffu, z[r], 1);
+        if (i == 0) {
+          zw = o5 * z[r] - h * zr;
+          fw = qx[r];
+        }
+      }
+      T ze = __shfl_down_sync(0xffffffffu, zw, 1), fe = __shfl_down_sync(0xffffffffu, fw, 1);
+      T zn = h * z[r] + h * z[r + 1], fn = h * (qy[r] + qy[r + 1]);
+      if (EDGE && i == nx - 1) {
+        ze = o5 * z[r] - h * zl;
+        fe = qx[r];
+      }
+      if (EDGE && j == ny - 1) {
+        zn = o5 * z[r] - h * z[r - 1];
+        fn = qy[r];
+      }
       const T sx = div_dx(ze - zw, dx, rdx), sy = div_dx(zn - zs, dx, rdx);
       const T div = div_dx(fe - fw, dx, rdx) + div_dx(fn - fs, dx, rdx);
-      a.W[(size_t)k * plane + off[r]] = (-div + u[r] * sx) + v[r] * sy;
+      if (out_lane && (!EDGE || j < ny)) W[(EDGE ? (size_t)j : (size_t)r) * nx + o0] = (-div + u[r] * sx) + v[r] * sy;
+      zs = zn;
+      fs = fn;
     }
   }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kVfWarps * 32, sizeof(T) == 4 ? 5 : 2) vert_flow_kernel(const VertFlowArgs<T> a, int n_strips) {
+  const int lane = threadIdx.x & 31;
+  const int gw = blockIdx.x * kVfWarps + (threadIdx.x >> 5);
+  const int strip = gw % n_strips, j0 = gw / n_strips * kVfRows;
+  if (j0 >= a.ny) return;  // uniform per warp
+  // rows j0 - 1 .. j0 + kVfRows and columns i of every lane inside the domain, no output on its border
+  const bool inner = j0 >= 1 && j0 + kVfRows < a.ny && strip >= 1 && (strip + 1) * kVfCols < a.nx;
+  if (inner)
+    vert_flow_march<T, false>(a, lane, strip, j0);
+  else
+    vert_flow_march<T, true>(a, lane, strip, j0);
 }
 
 // vert_flow version 2, incompressibility method (vert_flow_v2.py:40-57 with
@@ -619,7 +660,7 @@ __global__ void __launch_bounds__(kVfWarps * 32) vert_flow_incomp_kernel(const V
       un[r] = (more && in[r]) ? a.U[(size_t)(k + 1) * plane + off[r]] : T(0);
       vn[r] = (more && in[r]) ? a.V[(size_t)(k + 1) * plane + off[r]] : T(0);
     }
-    const T ddz = k > 0 ? a.lev[k] - a.lev[k - 1] : T(0);
+    const T ddz = a.ddz[k];
     const T wk = a.w[k];
     T z[R], dz[R];
 #pragma unroll
@@ -702,8 +743,10 @@ static int vert_flow_t(int nz, int ny, int nx, double dx, const void* U, const v
   a.dx = (T)dx;
   a.rdx = T(1) / a.dx;
   for (int k = 0; k < nz; ++k) {
-    a.lev[k] = (T)levels[k];
+    a.ddz[k] = k > 0 ? (T)levels[k] - (T)levels[k - 1] : T(0);
     a.w[k] = (T)vert_weight[k];
+    a.sw[k] = k > 0 ? a.sw[k - 1] + a.w[k] : a.w[k];
+    a.rsw[k] = T(1) / a.sw[k];  // host IEEE division in T
   }
   a.U = (const T*)U; a.V = (const T*)V; a.topg = (const T*)topg; a.thk = (const T*)thk; a.W = (T*)W;
   const int n_strips = (nx + kVfCols - 1) / kVfCols;

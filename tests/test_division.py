@@ -86,3 +86,13 @@ def test_markstein_division_by_cumulative_weights(nz, spacing):
             got = markstein_div(v32, b32, rb32)
             assert np.float32(got).tobytes() == np.float32(v32 / b32).tobytes(), (v32, b32)
             assert markstein_div64(float(v), b64, rb64) == float(v) / b64, (v, b64)
+
+
+def test_a_zero_numerator_keeps_its_sign():
+    """The kernels form the remainder as d q - a: zeros of either sign divide
+    to zeros of the same sign without a test (IEEE sums of signed zeros)."""
+    y, d = np.float32(0.02), np.float32(50.0)
+    for a in (np.float32(0.0), np.float32(-0.0)):
+        q = a * y
+        t = q * d + (-a)
+        assert np.signbit((-t) * y + q) == np.signbit(a) and (-t) * y + q == 0

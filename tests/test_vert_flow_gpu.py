@@ -70,6 +70,19 @@ def test_incompressibility_ragged_shapes_against_oracle(shape, dtype):
     np.testing.assert_array_equal(W.cpu().numpy(), ref.numpy())
 
 
+@pytest.mark.parametrize("shape", [(2, 7, 31), (3, 8, 60), (3, 13, 61), (2, 14, 62), (4, 18, 91), (10, 19, 120)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_inner_and_edge_segments_against_oracle(shape, dtype):
+    """Extents around the multiples of a warp's 30 columns and 6 rows, where a
+    strip or a segment just does or just does not touch the domain's border
+    (the kernel's border formulas are left out of the inner ones)."""
+    nz, ny, nx = shape
+    U, V, topg, thk, lv, w = _case(nz, ny, nx, nz * 100 + nx, dtype)
+    ref = O.vertical_velocity_kinematic(*(torch.as_tensor(a) for a in (U, V, topg, thk)), lv, w, 50.0)
+    W = K.vertical_velocity(dev(U), dev(V), dev(topg), dev(thk), lv.numpy(), w.numpy()[:, 0, 0], 50.0)
+    np.testing.assert_array_equal(W.cpu().numpy(), ref.numpy())
+
+
 def test_full_size_against_oracle():
     """1000 x 1000 x 10, FP32: bit-identical to the oracle."""
     U, V, topg, thk, lv, w = _case(10, 1000, 1000, 11, torch.float32)
