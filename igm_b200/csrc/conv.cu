@@ -105,7 +105,12 @@ __device__ __forceinline__ void set_err(int* err, int code) {
 // issues one bulk copy for its in-domain part; pixels and rows outside the
 // domain are zero-filled with shared-memory stores ("same" zero padding),
 // made visible to the tensor cores by a proxy fence before the arrival.
+// HALO_ONLY: past the right border only the one pixel that an output reads is
+// zero-filled (for callers whose pixels are the rows of the MMA: the pixels
+// beyond it reach only outputs that are not stored); a sum over pixels needs
+// them all.  Planes outside the domain are filled by the whole warp.
 // Lane 0 arrives on `bar` with the number of bytes the copies will deliver.
+template <bool HALO_ONLY = false>
 __device__ __forceinline__ void load_tile(const __nv_bfloat16* act, int H, int W, int c8, int b, int gy0, int rows,
                                           int gx0, int npx, unsigned char* dst, uint64_t* bar, int lane) {
   const int nplanes = rows * c8;
@@ -113,31 +118,27 @@ __device__ __forceinline__ void load_tile(const __nv_bfloat16* act, int H, int W
   const int xa = gx0 < 0 ? 0 : gx0;                // first in-domain pixel
   const int xb = gx0 + npx > W ? W : gx0 + npx;     // one past the last
   const uint32_t run = xb > xa ? (uint32_t)(xb - xa) * 16 : 0;
-  uint32_t mine = 0;
-  for (int p = lane; p < nplanes; p += 32) {
-    const int gy = gy0 + p / c8;
-    uint4* plane = reinterpret_cast<uint4*>(dst + (size_t)p * P);
-    const uint4 z = make_uint4(0, 0, 0, 0);
-    if (gy < 0 || gy >= H || run == 0) {
-      for (int q = 0; q < npx; ++q) plane[q] = z;
-    } else {
+  const int ra = run == 0 ? rows : (gy0 < 0 ? -gy0 : 0);                        // first in-domain row of the tile
+  const int rb = run == 0 ? rows : (gy0 + rows > H ? H - gy0 : rows);           // one past the last
+  const uint4 z = make_uint4(0, 0, 0, 0);
+  for (int q = lane; q < ra * c8 * npx; q += 32) reinterpret_cast<uint4*>(dst)[q] = z;
+  for (int q = rb * c8 * npx + lane; q < nplanes * npx; q += 32) reinterpret_cast<uint4*>(dst)[q] = z;
+  if (xa > gx0 || xb < gx0 + npx) {
+    const int xe = HALO_ONLY && xb + 1 < gx0 + npx ? xb + 1 : gx0 + npx;
+    for (int p = ra * c8 + lane; p < rb * c8; p += 32) {
+      uint4* plane = reinterpret_cast<uint4*>(dst + (size_t)p * P);
       for (int q = 0; q < xa - gx0; ++q) plane[q] = z;
-      for (int q = xb - gx0; q < npx; ++q) plane[q] = z;
-      mine += run;
+      for (int q = xb - gx0; q < xe - gx0; ++q) plane[q] = z;
     }
   }
-  uint32_t total = mine;
-  for (int o = 16; o > 0; o >>= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
   tc::fence_proxy_async_smem();
   __syncwarp();
-  if (lane == 0) tc::mbar_expect_tx(bar, total);
+  if (lane == 0) tc::mbar_expect_tx(bar, rb > ra ? (uint32_t)((rb - ra) * c8) * run : 0u);
   __syncwarp();
-  for (int p = lane; p < nplanes; p += 32) {
+  for (int p = ra * c8 + lane; p < rb * c8; p += 32) {
     const int gy = gy0 + p / c8, c = p % c8;
-    if (gy >= 0 && gy < H && run > 0) {
-      const __nv_bfloat16* src = act + ((((size_t)b * H + gy) * c8 + c) * W + xa) * 8;
-      tc::bulk_load(dst + (size_t)p * P + (size_t)(xa - gx0) * 16, src, run, bar);
-    }
+    const __nv_bfloat16* src = act + ((((size_t)b * H + gy) * c8 + c) * W + xa) * 8;
+    tc::bulk_load(dst + (size_t)p * P + (size_t)(xa - gx0) * 16, src, run, bar);
   }
 }
 
@@ -205,8 +206,8 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_kernel(const ConvA
       }
       const int txi = t % a.tiles_w, rest = t / a.tiles_w;
       const int tyi = rest % a.tiles_h, b = rest / a.tiles_h;
-      load_tile(a.x, a.H, a.W, C8_IN, b, tyi * R - 1, R + 2, txi * kTW - 1, kBoxW, smem + s * G::STAGE, &full[s],
-                lane);
+      load_tile<true>(a.x, a.H, a.W, C8_IN, b, tyi * R - 1, R + 2, txi * kTW - 1, kBoxW, smem + s * G::STAGE,
+                      &full[s], lane);
     }
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
@@ -463,6 +464,14 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_stack_kernel(const
           ok = false;
           break;
         }
+        unsigned char* st = smem + s * G::STAGE;
+        if (t == first(k) && lane == 0) {
+          // this layer's weights, on the barrier of its first tile (their buffer's last reader, layer
+          // k - 2, completed: the commit that released this stage covers every earlier MMA)
+          tc::mbar_expect_tx_only(&full[s], G::WBYTES);
+          tc::bulk_load(smem + G::OFF_W + (k & 1) * G::WBYTES, a.wpack[k], G::WBYTES, &full[s]);
+        }
+        __syncwarp();
         const int txi = t % a.tiles_w, rest = t / a.tiles_w;
         const int tyi = rest % a.tiles_h, b = rest / a.tiles_h;
         if (k > 0) {
@@ -478,7 +487,7 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_stack_kernel(const
                   got = false;
                   break;
                 }
-                __nanosleep(64);
+                __nanosleep(20);
               }
             }
           }
@@ -489,15 +498,7 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_stack_kernel(const
           }
           tc::fence_proxy_async_global();  // the acquired data is read next by the bulk-copy (async) proxy
         }
-        unsigned char* st = smem + s * G::STAGE;
-        if (t == first(k) && lane == 0) {
-          // this layer's weights, on the barrier of its first tile (their buffer's last reader, layer
-          // k - 2, completed: the commit that released this stage covers every earlier MMA)
-          tc::mbar_expect_tx_only(&full[s], G::WBYTES);
-          tc::bulk_load(smem + G::OFF_W + (k & 1) * G::WBYTES, a.wpack[k], G::WBYTES, &full[s]);
-        }
-        __syncwarp();
-        load_tile(src, a.H, a.W, 4, b, tyi * R - 1, R + 2, txi * kTW - 1, kBoxW, st, &full[s], lane);
+        load_tile<true>(src, a.H, a.W, 4, b, tyi * R - 1, R + 2, txi * kTW - 1, kBoxW, st, &full[s], lane);
       }
     }
   } else if (warp == 1) {
@@ -610,10 +611,8 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_stack_kernel(const
           ok = false;
           break;
         }
-        if (warp == 2 && lane == 0) {
-          __threadfence();
-          tc::st_release_gpu(a.flags + (size_t)k * per + t, a.epoch);
-        }
+        // (the release is cumulative over the barrier: it covers the stores of all eight warps)
+        if (warp == 2 && lane == 0) tc::st_release_gpu(a.flags + (size_t)k * per + t, a.epoch);
       }
     }
   }
@@ -1318,15 +1317,13 @@ extern "C" int igm_conv3x3_backward(int batch, int height, int width, const void
   return launch_status("conv3x3_bwd_kernel");
 }
 
-extern "C" int igm_conv3x3_stack(int batch, int height, int width, int nlayers, const void* x, void* const* outs,
+template <int R>
+static int stack_launch(int batch, int height, int width, int nlayers, const void* x, void* const* outs,
                                  const void* const* wpacks, const float* const* biases, int* flags, int epoch,
                                  float alpha, int* err, void* stream) {
-  constexpr int R = kRows;
   using G = ConvGeom<4, R>;
   constexpr uint32_t SMEM = G::OFF_W + 2 * G::WBYTES + 128 + 16 + 1024;
   static_assert(SMEM <= 232448, "shared memory");
-  IGM_CHECK_ARG(batch >= 1 && height >= 1 && width >= 1 && batch <= 65535, IGM_ERR_BAD_SHAPE,
-                "igm_conv3x3_stack: bad shape %dx%dx%d", batch, height, width);
   IGM_CHECK_ARG(nlayers >= 1 && nlayers <= kStackMax, IGM_ERR_BAD_SHAPE, "igm_conv3x3_stack: 1 .. %d layers",
                 kStackMax);
   IGM_CHECK_ARG(x && outs && wpacks && biases && flags && epoch != 0, IGM_ERR_BAD_ARGUMENT,
@@ -1369,8 +1366,38 @@ extern "C" int igm_conv3x3_stack(int batch, int height, int width, int nlayers, 
   return launch_status("conv3x3_stack_kernel");
 }
 
+// Output rows per tile of the stack.  While every tile of a layer can have an SM of its own, a layer
+// takes one tile's latency (load, MMAs, store, flag), which shrinks with the tile: the fewest rows
+// whose tiles still fit the SMs.  Above that the tiles queue, and the taller tile re-reads fewer halo
+// rows and hands over less often.  15 layers: 100 x 100 111 us with 8 rows, 62 with 2; 8 x 64 x 64 123
+// us with 8, 87 with 4; 1000 x 1000 the whole network is 4 % slower with 4 rows than with 8.
+static int stack_rows(int batch, int height, int width) {
+  const long long strips = (long long)batch * ((width + kTW - 1) / kTW);
+  for (int r = 2; r < kRows; r *= 2)
+    if (strips * ((height + r - 1) / r) <= sm_count()) return r;
+  return kRows;
+}
+
+extern "C" int igm_conv3x3_stack(int batch, int height, int width, int nlayers, const void* x, void* const* outs,
+                                 const void* const* wpacks, const float* const* biases, int* flags, int epoch,
+                                 float alpha, int* err, void* stream) {
+  IGM_CHECK_ARG(batch >= 1 && height >= 1 && width >= 1 && batch <= 65535, IGM_ERR_BAD_SHAPE,
+                "igm_conv3x3_stack: bad shape %dx%dx%d", batch, height, width);
+  switch (stack_rows(batch, height, width)) {
+    case 2:
+      return stack_launch<2>(batch, height, width, nlayers, x, outs, wpacks, biases, flags, epoch, alpha, err, stream);
+    case 4:
+      return stack_launch<4>(batch, height, width, nlayers, x, outs, wpacks, biases, flags, epoch, alpha, err, stream);
+    default:
+      return stack_launch<kRows>(batch, height, width, nlayers, x, outs, wpacks, biases, flags, epoch, alpha, err,
+                                 stream);
+  }
+}
+
 extern "C" size_t igm_conv3x3_stack_flags_len(int batch, int height, int width, int nlayers) {
-  return (size_t)nlayers * batch * ((width + kTW - 1) / kTW) * ((height + kRows - 1) / kRows);
+  if (batch < 1 || height < 1 || width < 1) return 0;
+  const int r = stack_rows(batch, height, width);
+  return (size_t)nlayers * batch * ((width + kTW - 1) / kTW) * ((height + r - 1) / r);
 }
 
 extern "C" int igm_conv1x1_wgrad(int batch, int height, int width, const void* x, const void* g, float* partials,

@@ -215,6 +215,14 @@ def test_conv_stack(B, H, W, nl, pingpong):
                 assert torch.equal(outs[k], ref[k]), k
 
 
+@pytest.mark.parametrize("B,H,W,pingpong", [(1, 1, 1, True), (1, 100, 100, True), (1, 101, 127, False), (1, 3, 129, True),
+                                            (8, 64, 64, True), (1, 72, 1000, False), (1, 73, 1000, True)])
+def test_conv_stack_tile_heights(B, H, W, pingpong):
+    """The stack at extents on both sides of its choice of rows per tile (2
+    and 4 while all tiles fit the SMs, else 8) and with ragged last tiles."""
+    test_conv_stack(B, H, W, 3, pingpong)
+
+
 @pytest.mark.parametrize("B,H,W,npart", [(1, 8, 128, 148), (2, 37, 300, 23), (1, 1000, 1000, 148)])
 def test_conv_backward_finishes_the_previous_layer(B, H, W, npart):
     """A fused backward call given the previous call's partial buffers also
