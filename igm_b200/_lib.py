@@ -101,6 +101,8 @@ SIGNATURES = {
     "igm_solver_begin": (I, [P, C.c_int64, P]),
     "igm_solver_iterate": (I, [I, C.POINTER(Grid), C.POINTER(Physics), C.POINTER(Fields), P, P, P, P, P, P, P, P,
                                C.POINTER(Adam), C.POINTER(EarlyStop), I, I, P, P, P, C.c_size_t, P]),
+    "igm_solver_solve": (I, [I, C.POINTER(Grid), C.POINTER(Physics), C.POINTER(Fields)] + [P] * 10
+                         + [C.POINTER(Adam), C.POINTER(EarlyStop), C.c_int64, I, P, P, P, C.c_size_t, P]),
     "igm_velocity_reduce": (I, [I, I, I, I, I, P, P, P, I, C.POINTER(C.c_double), P, P, P, P, P, P, P, P]),
     "igm_transport_step": (I, [I, I, I, D, P, P, P, P, P, P, P, P, P, D, P, I, D, D, P]),
     "igm_thk_surfaces": (I, [I, I, P, P, P, P, D, D, P]),

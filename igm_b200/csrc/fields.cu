@@ -23,6 +23,7 @@ struct VelArgs {
   T* us0;
   T* vs0;
   float* velomax;
+  int reads;  // some output is wanted; else the call only masks
 };
 
 template <typename T>
@@ -41,7 +42,7 @@ __global__ void __launch_bounds__(256) velocity_reduce_kernel(const VelArgs<T> a
         a.U[base + k * plane] = T(0);
         a.V[base + k * plane] = T(0);
       }
-    } else {
+    } else if (a.reads) {
       // the column's loads issued eight levels at a time (no store in this branch, so they need
       // not wait for one another); the sums in level order, as the reference's reduce_sum
       for (int k0 = 0; k0 < a.nz; k0 += 8) {
@@ -401,6 +402,7 @@ static int velocity_t(int batch, int nz, int ny, int nx, void* U, void* V, const
   for (int k = 0; k < nz; ++k) a.w[k] = (T)w[k];
   a.ubar = (T*)ubar; a.vbar = (T*)vbar; a.ub0 = (T*)ub0; a.vb0 = (T*)vb0; a.us0 = (T*)us0; a.vs0 = (T*)vs0;
   a.velomax = velomax;
+  a.reads = ubar || vbar || ub0 || vb0 || us0 || vs0 || velomax;
   if (velomax) {
     cudaError_t e = cudaMemsetAsync(velomax, 0, sizeof(float), st);
     if (e != cudaSuccess) {

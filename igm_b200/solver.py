@@ -43,29 +43,34 @@ class DeviceAdamSolver:
         dev = U.device
         g = L.make_grid(B, nz, ny, nx, dx, dzeta)
         ph = phys if isinstance(phys, L.Physics) else L.make_physics(phys)
-        U0, V0 = U4.clone(), V4.clone()
-        U1, V1 = torch.empty_like(U0), torch.empty_like(V0)
-        mU, mV, vU, vV = (torch.zeros_like(U0) for _ in range(4))
-        ctl = torch.zeros(C.sizeof(L.SolverCtl), dtype=torch.uint8, device=dev)
-        costs = torch.zeros(max(int(nbitmax), 1), dtype=torch.float64, device=dev)
+        # the start is read where it lies (iteration 0 reads it, later ones the two working pairs)
+        U4, V4 = (t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.clone() for t in (U4, V4))
+        U0, V0, U1, V1, mU, mV, vU, vV = (torch.empty_like(U4) for _ in range(8))
+        # control block and costs in one buffer: one copy to the host
+        nctl = (C.sizeof(L.SolverCtl) + 63) // 64 * 64
+        rec = torch.empty(nctl + 8 * max(int(nbitmax), 1), dtype=torch.uint8, device=dev)
+        ctl, costs = rec.data_ptr(), rec.data_ptr() + nctl
         es = L.EarlyStop()
         es.relative_min_delta, es.patience, es.enabled = float(relative_min_delta), int(patience), int(bool(early_stopping))
         wp, wn = workspace(dev).get(g, dev)
         f = fields_struct(*f2)
         st = L.stream_ptr()
         lib = L.lib()
-        L.check(lib.igm_solver_begin(L.ptr(ctl), int(self.iterations), st), "igm_solver_begin")
         if nbitmax > 0:
-            rc = lib.igm_solver_iterate(L.dtype_code(U.dtype), C.byref(g), C.byref(ph), C.byref(f),
-                                        L.ptr(U0), L.ptr(V0), L.ptr(U1), L.ptr(V1), L.ptr(mU), L.ptr(mV), L.ptr(vU),
-                                        L.ptr(vV), C.byref(self.adam), C.byref(es), int(nbitmax), int(nbitmax),
-                                        L.ptr(ctl), L.ptr(costs), wp, wn, st)
-            L.check(rc, "igm_solver_iterate")
-        hc = L.SolverCtl.from_buffer_copy(ctl.cpu().numpy().tobytes())
+            rc = lib.igm_solver_solve(L.dtype_code(U.dtype), C.byref(g), C.byref(ph), C.byref(f), L.ptr(U4), L.ptr(V4),
+                                      L.ptr(U0), L.ptr(V0), L.ptr(U1), L.ptr(V1), L.ptr(mU), L.ptr(mV), L.ptr(vU),
+                                      L.ptr(vV), C.byref(self.adam), C.byref(es), int(self.iterations), int(nbitmax),
+                                      ctl, costs, wp, wn, st)
+            L.check(rc, "igm_solver_solve")
+        else:
+            L.check(lib.igm_solver_begin(ctl, int(self.iterations), st), "igm_solver_begin")
+            U0, V0 = U4.clone(), V4.clone()
+        host = rec.cpu().numpy()
+        hc = L.SolverCtl.from_buffer_copy(host[:nctl].tobytes())
         n = int(hc.iter)
         self.iterations += n
         self.last_status = int(hc.status)
-        self.last_costs = costs[:n].cpu().numpy()
+        self.last_costs = host[nctl:nctl + 8 * n].view(np.float64).copy()
         if hc.status != 0:
             raise L.IgmError(hc.status, f"solver stopped at iteration {n}: non-finite energy")
         Ur, Vr = (U0, V0) if n % 2 == 0 else (U1, V1)

@@ -201,6 +201,17 @@ IGM_API int igm_solver_iterate(int dtype, const igm_grid* grid, const igm_physic
                        igm_solver_ctl* ctl, double* costs, void* workspace, size_t workspace_bytes,
                        void* stream);
 
+/* A whole solve: igm_solver_begin and max_iter iterations from the start Uin,
+ * Vin (not modified) with zero moments.  U0 .. vV are scratch and need no
+ * initial values.  After ctl->iter iterations (read back by the caller) the
+ * result is in U1, V1 when that number is odd and in U0, V0 when it is even;
+ * costs holds that many values. */
+IGM_API int igm_solver_solve(int dtype, const igm_grid* grid, const igm_physics* phys, const igm_fields* fields,
+                     const void* Uin, const void* Vin, void* U0, void* V0, void* U1, void* V1, void* mU, void* mV,
+                     void* vU, void* vV, const igm_adam* adam, const igm_early_stop* early_stop,
+                     int64_t adam_iterations, int max_iter, igm_solver_ctl* ctl, double* costs, void* workspace,
+                     size_t workspace_bytes, void* stream);
+
 /* ---------------------------------------------------------------------------
  * Velocity post-processing: optional mask U,V = where(thk > 0, U, 0)
  * (solve.py:116-117, emulate.py:143-144), then velbase = U[0],

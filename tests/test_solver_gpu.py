@@ -139,3 +139,42 @@ def test_fp32_solver_matches_fp32_oracle_to_1e5():
     print(f"one iteration: device FP32 vs oracle FP32 {e:.3e}")
     assert e <= 1e-5, e
     np.testing.assert_allclose(c, cref, rtol=1e-5)
+
+
+@pytest.mark.parametrize("n", [0, 1, 2, 5])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_start_is_read_in_place(n, offset):
+    """A solve reads its start where it lies (copied when it is not 16-byte
+    aligned) and leaves it unchanged, whatever the number of iterations'
+    parity; without ice the gradient and the step are zero.  Against the
+    solve in single iterations' entry point from copies and zeroed moments."""
+    import ctypes as C
+    from igm_b200.kernels import fields_struct, workspace
+    st = O.valley_glacier(40, 36, 100.0, seed=4, varying_coeffs=True)
+    f = [dev(st[k], torch.float32) for k in ["thk", "usurf", "arrhenius", "slidingco"]]
+    nz = 6
+    dz = O.compute_zeta_dzeta(O.compute_levels(nz, 4.0))[1].numpy()
+    rng = np.random.default_rng(3)
+    base = torch.as_tensor(rng.normal(20, 10, (2, nz * 40 * 36 + 1)).astype(np.float32)).cuda()
+    U, V = (base[i, offset:offset + nz * 40 * 36].view(nz, 40, 36) for i in range(2))
+    U *= f[0] > 0
+    V *= f[0] > 0
+    keep = base.clone()
+    s = DeviceAdamSolver()
+    s.iterations = 3
+    Ur, Vr, costs = s.solve(U, V, *f, 100.0, dz, nbitmax=n, early_stopping=False)
+    assert torch.equal(base, keep) and len(costs) == n and s.iterations == 3 + n
+    g, ph, fs = L.make_grid(1, nz, 40, 36, 100.0, dz), L.make_physics(), fields_struct(*f)
+    W = [U.clone(), V.clone(), torch.empty_like(U), torch.empty_like(V)] + [torch.zeros_like(U) for _ in range(4)]
+    ctl = torch.zeros(C.sizeof(L.SolverCtl), dtype=torch.uint8, device="cuda")
+    cs = torch.zeros(max(n, 1), dtype=torch.float64, device="cuda")
+    es = L.EarlyStop()
+    wp, wn = workspace("cuda").get(g, U.device)
+    lib, stream = L.lib(), L.stream_ptr()
+    L.check(lib.igm_solver_begin(L.ptr(ctl), 3, stream))
+    L.check(lib.igm_solver_iterate(0, C.byref(g), C.byref(ph), C.byref(fs), *[L.ptr(w) for w in W], C.byref(s.adam),
+                                   C.byref(es), n, max(n, 1), L.ptr(ctl), L.ptr(cs), wp, wn, stream))
+    ice = f[0] > 0
+    for got, ref in zip((Ur, Vr), W[2 * (n % 2):2 * (n % 2) + 2]):
+        assert torch.equal(got, torch.where(ice, ref, torch.zeros_like(ref)))
+    np.testing.assert_array_equal(costs, cs.cpu().numpy()[:n])
