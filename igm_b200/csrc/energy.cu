@@ -261,6 +261,7 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
   using SmemT = StencilSmem<T, TYP, MODE>;
   // STD: the default physics (Glen n = 3, Weertman m = 3, gravitational energy not forced
   // negative), fixed at compile time so that its branches and generic powers drop out
+  constexpr bool kSkip = STD;  // bare warps skip their layers
   const bool glen3 = STD || a.glen3, weert3 = STD || a.weert3, fnge = !STD && a.fnge;
   constexpr int TYC = 2 * TYP;  // cell rows per tile
   constexpr int NT = kCW * TYP;
@@ -511,6 +512,12 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
     const long long obase = ((long long)g.b * nz) * (long long)plane +
                             (long long)(g.j0 - 1 + R0) * nx + (g.i0 - 1 + tx);
 
+    // No ice in this warp's cells (warp-uniform): their shear and gravity energies and gradients are
+    // exactly zero, whatever finite velocities a level holds, so its layers are skipped.
+    // Half of a valley, and more of most domains, is such ground.  Half of it ice: energy and adjoint at
+    // 1000 x 1000 x 10 98 -> 90 us, energy 51 -> 47; FP64 at 400 x 400 43.2 -> 34.6 and 26.8 -> 22.7.
+    const bool bare = kSkip && nz > 1 && __all_sync(0xffffffffu, thks.x == T(0) && thks.y == T(0));
+    bool pending = true;  // the adjoint awaiting its flush may be non-zero (warp-uniform)
     P e_sh = zero, eGu = zero, eGv = zero, e_slid = zero, e_gf = zero;
     // previous level's corner sums, pending adjoint of the previous level
     P pSu = zero, pSv = zero, pXu = zero, pYu = zero, pXv = zero, pYv = zero;
@@ -593,6 +600,35 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
       P cSu, cXu, cYu, cSv, cXv, cYv;
       level_q(SM.N[nb][0], cSu, cXu, cYu);
       level_q(SM.N[nb][1], cSv, cXv, cYv);
+      if (kSkip && !FIRST && bare) {
+        // Idle while every value is far from overflowing the products below (and no NaN): then they
+        // are finite, and zero times them is zero.
+        const P big = {fabs(cSu.x) + fabs(cXu.x) + fabs(cYu.x) + fabs(cSv.x) + fabs(cXv.x) + fabs(cYv.x),
+                       fabs(cSu.y) + fabs(cXu.y) + fabs(cYu.y) + fabs(cSv.y) + fabs(cXv.y) + fabs(cYv.y)};
+        if (__all_sync(0xffffffffu, big.x < T(1e10) && big.y < T(1e10))) {
+          if (GRAD) {
+            if (pending) {
+              flush(k - 1, gSu, gXu, gYu, 0, partU);
+              flush(k - 1, gSv, gXv, gYv, 1, partV);
+              gSu = zero; gXu = zero; gYu = zero; gSv = zero; gXv = zero; gYv = zero;
+              pending = false;
+            } else {
+              partU = zero;
+              partV = zero;
+              SM.Down[(k - 1) & 1][0][ty][tx] = T(0);
+              SM.Down[(k - 1) & 1][1][ty][tx] = T(0);
+            }
+          }
+          pSu = cSu; pSv = cSv; pXu = cXu; pYu = cYu; pXv = cXv; pYv = cYv;
+          st_m2 = st_m1;
+          st_m1 = nb;
+          if (++cons_st == kStages) {
+            cons_st = 0;
+            cons_ph ^= 1u;
+          }
+          return;
+        }
+      }
       // gravity of level k (weight dzeta[k-1] + dzeta[k]) enters its pending adjoint directly
       const T wk = a.wgrav[k];
       if (!fnge) {
@@ -704,6 +740,7 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
           flush(k - 1, gSv, gXv, gYv, 1, partV);
         }
         gSu = hSu; gXu = hXu; gYu = hYu; gSv = hSv; gXv = hXv; gYv = hYv;
+        pending = true;
       }
       pSu = cSu; pSv = cSv; pXu = cXu; pYu = cYu; pXv = cXv; pYv = cYv;
       st_m2 = st_m1;

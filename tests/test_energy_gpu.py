@@ -157,3 +157,44 @@ def test_other_physics_against_oracle(n, m, fnge):
                                atol=1e-10 * float(cost.abs()))
     assert rel_l2(dU.cpu().numpy(), gU.numpy()) < 1e-10
     assert rel_l2(dV.cpu().numpy(), gV.numpy()) < 1e-10
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("ice_rows,value", [((0, 0), 0.0), ((20, 21), 0.0), ((16, 48), 1e12), ((16, 48), float("nan")),
+                                            ((16, 48), float("inf"))])
+def test_bare_ground(dtype, ice_rows, value):
+    """Cells without ice skip their layers: none, one or a third of the rows
+    under ice, moving ground everywhere (sliding acts without ice too), and one
+    off-ice node (row 60, level 2) with a value whose products overflow or are
+    not finite, which must not be skipped.  Against autograd of the oracle in
+    FP64; tolerances as above (2e-5 for the FP32 gradient against FP64)."""
+    ny, nx, nz = 70, 66, 5
+    st = O.valley_glacier(ny, nx, 100.0, seed=5, varying_coeffs=True)
+    rng = np.random.default_rng(6)
+    thk = np.zeros((ny, nx))
+    thk[ice_rows[0]:ice_rows[1]] = rng.uniform(50, 150, (ice_rows[1] - ice_rows[0], nx))
+    U, V = rng.normal(20, 10, (nz, ny, nx)), rng.normal(0, 10, (nz, ny, nx))
+    if value:
+        U[2, 60, 33] = value
+    np_dt = np.float32 if dtype == torch.float32 else np.float64
+    f64 = [np.asarray(a, np_dt).astype(np.float64) for a in (thk, st["topg"] + thk, st["arrhenius"], st["slidingco"])]
+    U, V = U.astype(np_dt), V.astype(np_dt)
+    dz = O.compute_zeta_dzeta(O.compute_levels(nz, 4.0).double())[1]
+    ns = (ny - 1) * (nx - 1)
+    terms, dU, dV = K.energy(dev(U, dtype), dev(V, dtype), *[dev(a, dtype) for a in f64], 100.0, dz.numpy(), grad=True,
+                             grad_scale=1.0 / ns)
+    terms2, _, _ = K.energy(dev(U, dtype), dev(V, dtype), *[dev(a, dtype) for a in f64], 100.0, dz.numpy())
+    assert np.array_equal(terms.cpu().numpy(), terms2.cpu().numpy(), equal_nan=True)
+    if not np.isfinite(value):
+        assert not bool(torch.isfinite(terms.sum())) and not bool(torch.isfinite(dU).all())
+        ok = torch.ones((ny, nx), dtype=torch.bool)
+        ok[58:63, 31:36] = False
+        assert bool(torch.isfinite(dU.cpu()[:, ok]).all())
+        return
+    cost, means, gU, gV = O.energy_and_grad(torch.as_tensor(U).double(), torch.as_tensor(V).double(),
+                                            *[torch.as_tensor(a) for a in f64], 100.0, dz)
+    tol = 1e-11 if dtype == torch.float64 else 2e-5
+    np.testing.assert_allclose(terms.cpu().numpy() / ns, [float(m) for m in means], rtol=tol,
+                               atol=tol * max(abs(float(m)) for m in means))
+    assert rel_l2(dU.cpu().numpy(), gU.numpy()) < tol
+    assert rel_l2(dV.cpu().numpy(), gV.numpy()) < tol
