@@ -181,6 +181,8 @@ struct StencilArgs {
   T* dU;
   T* dV;
   T grad_scale;
+  const T* grad_out;   // when set: the scale is *grad_out / grad_count, read on the device
+  double grad_count;
   // solver mode; Uin, Vin (else NULL): the start of a solve, read by iteration 0 in place of U0, V0,
   // with the moments taken as zero there, not read
   const T* Uin;
@@ -417,6 +419,7 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
 #pragma unroll 1
   for (int q = 0; q < kAhead; ++q) issue_next();
 
+  const T gscale = MODE == kGradient && a.grad_out ? (T)((double)__ldg(a.grad_out) / a.grad_count) : a.grad_scale;
   const T half = T(0.5), quarter = T(0.25);
   const P H = two(half), Q4 = two(quarter), zero = two(T(0));
   const P HI = two(half * a.inv_dx);
@@ -504,7 +507,7 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
     const P egc = thks * two(a.Kg * T(0.125));
     // adjoint constants (grad_scale folded in; zero for cells outside the domain, whose
     // contributions then vanish without masking)
-    const P okm = sel(cok[0], cok[1], two(a.grad_scale), zero);
+    const P okm = sel(cok[0], cok[1], two(gscale), zero);
     const P gshc = esc * okm;                // dE/d(bq sr2w) per unit dzeta
     const P gxc = egc * ssx * okm, gyc = egc * ssy * okm;  // dE/dS, dE/dSV per unit gravity weight
     const P csg = cs * okm * Q4;             // sliding: dE/dS = csg N^(s/2-1) (Us + tb sbx)
@@ -1063,7 +1066,8 @@ static int launch_stencil(const StencilArgs<T>& s, const StencilMaps& maps, bool
 
 template <typename T>
 static int energy_t(const igm_grid* g, const igm_physics* ph, const igm_fields* f, const void* U, const void* V,
-                    void* dU, void* dV, double grad_scale, double* terms, void* ws, size_t wsb, cudaStream_t st) {
+                    void* dU, void* dV, double grad_scale, double* terms, void* ws, size_t wsb, cudaStream_t st,
+                    const void* grad_out = nullptr, double grad_count = 1.0) {
   StencilArgs<T> s{};
   fill_common(s, g, ph, f);
   s.U0 = (T*)U;
@@ -1071,6 +1075,8 @@ static int energy_t(const igm_grid* g, const igm_physics* ph, const igm_fields* 
   s.dU = (T*)dU;
   s.dV = (T*)dV;
   s.grad_scale = (T)grad_scale;
+  s.grad_out = (const T*)grad_out;
+  s.grad_count = grad_count;
   s.terms = terms;
   int rc = bind_workspace(ws, wsb, g, &s.counter, &s.partials);
   if (rc) return rc;
@@ -1247,6 +1253,25 @@ extern "C" int igm_energy(int dtype, const igm_grid* grid, const igm_physics* ph
     return energy_t<double>(grid, phys, fields, U, V, dU, dV, grad_scale, terms, workspace, workspace_bytes, st);
   set_error("igm_energy: unknown dtype %d", dtype);
   return IGM_ERR_BAD_ARGUMENT;
+}
+
+extern "C" int igm_energy_backward(int dtype, const igm_grid* grid, const igm_physics* phys, const igm_fields* fields,
+                                   const void* U, const void* V, void* dU, void* dV, const void* grad_out,
+                                   double grad_count, double* terms, void* workspace, size_t workspace_bytes,
+                                   void* stream) {
+  int rc = check_grid(grid);
+  if (rc) return rc;
+  IGM_CHECK_ARG(phys && fields && U && V && dU && dV && grad_out && terms && grad_count != 0, IGM_ERR_BAD_ARGUMENT,
+                "igm_energy_backward: NULL argument or zero count");
+  IGM_CHECK_ARG(fields->thk && fields->usurf && fields->arrhenius && fields->slidingco, IGM_ERR_BAD_ARGUMENT,
+                "igm_energy_backward: NULL field");
+  IGM_CHECK_ARG(dtype == IGM_F32 || dtype == IGM_F64, IGM_ERR_BAD_ARGUMENT, "igm_energy_backward: unknown dtype %d", dtype);
+  cudaStream_t st = as_stream(stream);
+  if (dtype == IGM_F32)
+    return energy_t<float>(grid, phys, fields, U, V, dU, dV, 0.0, terms, workspace, workspace_bytes, st, grad_out,
+                           grad_count);
+  return energy_t<double>(grid, phys, fields, U, V, dU, dV, 0.0, terms, workspace, workspace_bytes, st, grad_out,
+                          grad_count);
 }
 
 extern "C" int igm_solver_begin(igm_solver_ctl* ctl, int64_t adam_iterations, void* stream) {

@@ -47,9 +47,11 @@ def fields_struct(thk, usurf, arrhenius, slidingco) -> L.Fields:
 
 
 def energy(U, V, thk, usurf, arrhenius, slidingco, dx, dzeta, phys=None, grad=False, grad_scale=1.0,
-           terms_out=None):
+           terms_out=None, grad_out=None, grad_count=1.0):
     """Energy sums (device float64 [3]: shear, sliding, gravity) and optionally
-    grad_scale * d(sum)/d(U,V).  U, V: [B, Nz, Ny, Nx] or [Nz, Ny, Nx]."""
+    grad_scale * d(sum)/d(U,V).  U, V: [B, Nz, Ny, Nx] or [Nz, Ny, Nx].  With
+    ``grad_out`` (a device tensor of one value, U's dtype) the gradient's scale
+    is grad_out / grad_count, read on the device."""
     squeeze = U.dim() == 3
     if squeeze:
         U, V = U[None], V[None]
@@ -62,9 +64,17 @@ def energy(U, V, thk, usurf, arrhenius, slidingco, dx, dzeta, phys=None, grad=Fa
     dV = torch.empty_like(V) if grad else None
     wp, wn = workspace(U.device).get(g, U.device)
     f = fields_struct(thk, usurf, arrhenius, slidingco)
-    rc = L.lib().igm_energy(L.dtype_code(U.dtype), C.byref(g), C.byref(ph), C.byref(f), L.ptr(U), L.ptr(V),
-                            L.ptr(dU), L.ptr(dV), float(grad_scale), L.ptr(terms), wp, wn, L.stream_ptr())
-    L.check(rc, "igm_energy")
+    if grad and grad_out is not None:
+        if grad_out.dtype != U.dtype or grad_out.numel() != 1:
+            raise ValueError("energy: grad_out must be one value of U's dtype")
+        rc = L.lib().igm_energy_backward(L.dtype_code(U.dtype), C.byref(g), C.byref(ph), C.byref(f), L.ptr(U), L.ptr(V),
+                                         L.ptr(dU), L.ptr(dV), L.ptr(grad_out), float(grad_count), L.ptr(terms), wp, wn,
+                                         L.stream_ptr())
+        L.check(rc, "igm_energy_backward")
+    else:
+        rc = L.lib().igm_energy(L.dtype_code(U.dtype), C.byref(g), C.byref(ph), C.byref(f), L.ptr(U), L.ptr(V),
+                                L.ptr(dU), L.ptr(dV), float(grad_scale), L.ptr(terms), wp, wn, L.stream_ptr())
+        L.check(rc, "igm_energy")
     if squeeze and grad:
         dU, dV = dU[0], dV[0]
     return terms, dU, dV

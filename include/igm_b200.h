@@ -155,6 +155,13 @@ IGM_API int igm_energy(int dtype, const igm_grid* grid, const igm_physics* phys,
                const void* U, const void* V, void* dU, void* dV, double grad_scale, double* terms,
                void* workspace, size_t workspace_bytes, void* stream);
 
+/* igm_energy with gradients whose scale lies on the device: grad_scale =
+ * *grad_out / grad_count (grad_out: one value of the dtype; the division in
+ * double), as the backward of cost = sum(terms) / grad_count needs it. */
+IGM_API int igm_energy_backward(int dtype, const igm_grid* grid, const igm_physics* phys, const igm_fields* fields,
+                        const void* U, const void* V, void* dU, void* dV, const void* grad_out, double grad_count,
+                        double* terms, void* workspace, size_t workspace_bytes, void* stream);
+
 /* Same computation and results as igm_energy, for callers that cannot
  * allocate device memory: a host model that has already handed all device
  * memory to its own pool, or code that must not call cudaMalloc/cudaFree

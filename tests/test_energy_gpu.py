@@ -198,3 +198,21 @@ def test_bare_ground(dtype, ice_rows, value):
                                atol=tol * max(abs(float(m)) for m in means))
     assert rel_l2(dU.cpu().numpy(), gU.numpy()) < tol
     assert rel_l2(dV.cpu().numpy(), gV.numpy()) < tol
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("gout", [1.0, -0.37, 0.0])
+def test_backward_scale_on_the_device(dtype, gout):
+    """The autograd backward, whose scale is divided on the device, against
+    the gradient with the same scale given by the host: the same bits."""
+    from igm_b200.energy import iceflow_energy
+    ny, nx, nz = 33, 41, 4
+    st = O.valley_glacier(ny, nx, 100.0, seed=7, varying_coeffs=True)
+    rng = np.random.default_rng(8)
+    f = [dev(st[k], dtype) for k in ["thk", "usurf", "arrhenius", "slidingco"]]
+    dz = O.compute_zeta_dzeta(O.compute_levels(nz, 4.0).double())[1].numpy()
+    U, V = (dev(rng.normal(5, 9, (nz, ny, nx)), dtype).requires_grad_(True) for _ in range(2))
+    g = torch.tensor(gout, dtype=dtype, device="cuda")
+    dU, dV = torch.autograd.grad(iceflow_energy(U, V, *f, 100.0, dz), [U, V], grad_outputs=g)
+    _, rU, rV = K.energy(U.detach(), V.detach(), *f, 100.0, dz, grad=True, grad_scale=float(g) / ((ny - 1) * (nx - 1)))
+    assert torch.equal(dU, rU) and torch.equal(dV, rV)
