@@ -809,29 +809,32 @@ def assimilation_cpu(args, crop):
             "sample": f"one optimize_update iteration of the oracle on a {crop}x{crop} crop (second of two), "
                       f"scaled by ({args.size}/{crop})^2; emulator retraining not included"}
 
-def roofline_conv(conv_ms, size, peaks, layers=15):
-    """The forward conv stack (15 layers of 3x3 conv, 32 -> 32 channels, in one
-    launch): algorithmic bytes per launch = per layer one read of the input
-    activation and one write of the output, 2 x 64 B per pixel."""
+def roofline_conv(conv_ms, size, peaks, layers=16):
+    """The forward convolutions of an inference in one launch (the chain: the
+    first layer, 16-channel split input, and 15 layers of 32 -> 32 channels, two
+    per pass over memory): multiplications and additions of the 3x3 taps
+    against the measured bf16 rate; algorithmic bytes = per pass one read of its
+    input (32 B per pixel for the first, then 64) and one write of 64 B."""
     if not conv_ms:
         return None
     t = float(np.mean(conv_ms)) / 1e3
-    byts = layers * 2 * 64 * size * size
-    achieved = byts / t / 1e9
-    peak = peaks.get("hbm_gbs", 6650.0)
-    # DRAM traffic of one launch from the committed ncu capture of the same launch (15 layers,
+    byts = (layers // 2 * 128 - 32) * size * size
+    achieved = 2 * 9 * 32 * (16 + 32 * (layers - 1)) * size * size / t / 1e12
+    peak = peaks.get("bf16_tflops", 1590.0)
+    # DRAM traffic of one launch from the committed ncu capture of the same launch (16 layers,
     # batch 1 x 1000 x 1000), scaled to this launch's pixels
     traffic = None
-    prof = os.path.join(ROOT, "profiles", "conv3x3_stack_15x1000x1000.txt")
+    prof = os.path.join(ROOT, "profiles", "conv3x3_chain_16x1000x1000.txt")
     if os.path.exists(prof):
         for line in open(prof):
             if line.startswith("dram_bytes_per_launch:"):
                 traffic = round(float(line.split(":")[1]) * (size * size) / (1000 * 1000))
-    return {"kernel": f"conv3x3_stack_kernel<8> (tcgen05, {layers} layers of cin 32 per launch)", "bound": "hbm",
-            "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s", "frac": round(achieved / peak, 4),
+    return {"kernel": f"conv3x3_chain_kernel (tcgen05, {layers} layers per launch, two per pass over memory)",
+            "bound": "tensor",
+            "achieved": round(achieved, 1), "peak": peak, "unit": "TFLOP/s", "frac": round(achieved / peak, 4),
             "traffic": traffic, "algorithmic_bytes": byts, "avg_launch_us": round(t * 1e6, 2),
             "avg_layer_us": round(t * 1e6 / layers, 2), "launches": len(conv_ms),
-            "peak_source": "MEASURED_PEAKS.json hbm_gbs (of measured)" if "hbm_gbs" in peaks else "fallback"}
+            "peak_source": "MEASURED_PEAKS.json bf16_tflops (of measured)" if "bf16_tflops" in peaks else "fallback"}
 
 
 def plain_run_100x100(args, cpu_steps=2, gpu_max_steps=3000, gpu_max_s=40.0):
@@ -1298,7 +1301,7 @@ def main():
             "fallback_checks": res["fallback_checks"], "fallbacks": res["fallbacks"],
             "years_per_time_step_emulated": em["years"] / (K * TIME_STEPS_PER_STEP),
             "years_per_time_step_plain": sv["years"] / (K * TIME_STEPS_PER_STEP),
-            "roofline": roofline_conv(conv_ms, args.size, peaks, layers=15),
+            "roofline": roofline_conv(conv_ms, args.size, peaks),
             "clocks": clocks, "gpu_launches": int(launches), "e2e": e2e}
     if rank == 0:
         if "plain_100x100" in det:

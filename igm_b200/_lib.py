@@ -120,6 +120,9 @@ SIGNATURES = {
     "igm_conv3x3_backward": (I, [I, I, I, P, P, P, P, P, P, I, C.c_float, P, P, P, P, P, P]),
     "igm_conv3x3_stack": (I, [I, I, I, I, P, P, P, P, P, I, C.c_float, P, P]),
     "igm_conv3x3_stack_flags_len": (C.c_size_t, [I, I, I, I]),
+    "igm_conv3x3_chain": (I, [I, I, I, I, I, P, P, P, P, P, P, I, C.c_float, P, P]),
+    "igm_conv3x3_chain_flags_len": (C.c_size_t, [I, I, I, I]),
+    "igm_conv3x3_chain_pays": (I, [I, I, I, I]),
     "igm_conv_sm_count": (I, []),
     "igm_conv3x3_wgrad_partial_len": (C.c_size_t, [I]),
     "igm_cnn_param_count": (C.c_size_t, [I, I, I]),

@@ -149,8 +149,10 @@ class CNN:
                 b["dbpart2"] = [torch.zeros((npart, F), dtype=torch.float32, device=d) for _ in range(2)]
                 hl = int(L.lib().igm_cnn_head_partial_len(self.nz))
                 b["hpart"] = torch.empty((2 * npart, hl), dtype=torch.float32, device=d)
-            nst = max(self.L - 1, 1)
-            b["flags"] = torch.zeros(int(L.lib().igm_conv3x3_stack_flags_len(B, h, w, nst)), dtype=torch.int32, device=d)
+            b["chain"] = self.L >= 2 and bool(L.lib().igm_conv3x3_chain_pays(B, h, w, int(train)))
+            nfl = (L.lib().igm_conv3x3_chain_flags_len(B, h, w, self.L // 2 * 2) if b["chain"]
+                   else L.lib().igm_conv3x3_stack_flags_len(B, h, w, max(self.L - 1, 1)))
+            b["flags"] = torch.zeros(int(nfl), dtype=torch.int32, device=d)
             self._bufs[key] = b
         return b
 
@@ -176,11 +178,14 @@ class CNN:
         head -- all convolutions on the tensor cores; U, V into buf."""
         lib, st = L.lib(), L.stream_ptr()
         acts = buf["acts"]
-        rc = lib.igm_conv3x3(0, B, h, w, 16, _p(buf["X"]), self._wf(0), self._b(0), None, _p(acts[0]), None, 0,
-                             self.alpha, _p(self.err), st)
-        L.check(rc, "igm_conv3x3 layer 0")
-        x = acts[0]
-        if self.L > 1:
+        if buf["chain"]:
+            x = self._forward_chain(buf, B, h, w, keep_acts, st)
+        else:
+            rc = lib.igm_conv3x3(0, B, h, w, 16, _p(buf["X"]), self._wf(0), self._b(0), None, _p(acts[0]), None, 0,
+                                 self.alpha, _p(self.err), st)
+            L.check(rc, "igm_conv3x3 layer 0")
+            x = acts[0]
+        if self.L > 1 and not buf["chain"]:
             # the 32-channel layers 1 .. L-1 in one launch (igm_conv3x3_stack)
             n = self.L - 1
             ys = [acts[l] if keep_acts else acts[l % 2] for l in range(1, self.L)]
@@ -205,6 +210,35 @@ class CNN:
                                       _p(thk_mask), st)
         L.check(rc, "igm_cnn_head_forward")
         return buf["U"], buf["V"]
+
+    def _forward_chain(self, buf, B, h, w, keep_acts, st):
+        """The 3x3 layers two per pass (igm_conv3x3_chain), an odd last one by
+        itself; returns the last activation."""
+        lib, acts = L.lib(), buf["acts"]
+        n = self.L // 2
+        outs = [acts[2 * k + 1] if keep_acts else acts[k % 2] for k in range(n)]
+        mids = (C.c_void_p * n)(*[_p(acts[2 * k]) if keep_acts else None for k in range(n)])
+        wps = (C.c_void_p * (2 * n))(*[self._wf(l) for l in range(2 * n)])
+        bs = (C.c_void_p * (2 * n))(*[self._b(l) for l in range(2 * n)])
+        self._epoch = self._epoch % 2147483646 + 1
+        hook = self.event_hook if not keep_acts else None
+        if hook is not None:
+            ev = (torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True))
+            ev[0].record()
+        rc = lib.igm_conv3x3_chain(B, h, w, 2 * n, 16, _p(buf["X"]), mids, (C.c_void_p * n)(*[_p(y) for y in outs]), wps,
+                                   bs, _p(buf["flags"]), self._epoch, self.alpha, _p(self.err), st)
+        L.check(rc, "igm_conv3x3_chain")
+        if hook is not None:
+            ev[1].record()
+            hook.append(ev)
+        x = outs[-1]
+        if self.L % 2:
+            y = acts[self.L - 1] if keep_acts else acts[n % 2]
+            rc = lib.igm_conv3x3(0, B, h, w, F, _p(x), self._wf(self.L - 1), self._b(self.L - 1), None, _p(y), None, 0,
+                                 self.alpha, _p(self.err), st)
+            L.check(rc, "igm_conv3x3 last layer")
+            x = y
+        return x
 
     # ---- backward ----------------------------------------------------------
     def backward(self, buf, B, h, w, dU, dV, field_grad=None, param_grads=True):

@@ -624,6 +624,482 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_stack_kernel(const
 }
 
 // ---------------------------------------------------------------------------
+// forward of a chain of layers, two layers per pass over memory
+// ---------------------------------------------------------------------------
+// A layer alone reads and writes 64 B per pixel and multiplies 18,432 times:
+// run one by one the layers move more bytes between the SMs and memory than the
+// tensor cores take time for (26 us per 1000 x 1000 layer against 11 us of
+// math).  Here a pass over memory computes two layers (A, then B): a CTA walks
+// down a strip of 126 output columns, row by row, and
+//   * layer A's input rows arrive in a ring (bulk copies of 130 pixels),
+//   * input row i adds into the accumulators of A's rows i-2, i-1, i (kernel
+//     rows 2, 1, 0; as in conv3x3_kernel one MMA of N = 96 per column tap and
+//     K step, here over a ring of 8 row accumulators in TMEM),
+//   * A's finished rows go through bias and LeakyReLU into a second ring in
+//     shared memory in the operand layout (128 pixels: the strip and one pixel
+//     on each side, zero outside the domain), and to memory only when the caller
+//     keeps the activations,
+//   * layer B reads that ring in the same way, 8 more row accumulators, and its
+//     rows are stored.
+// No row is read twice but at the strips' borders (4 of 130 columns) and the
+// four rows above and below a piece.  Each output sums its products in the order of
+// conv3x3_kernel, so the results are the same bits.
+//
+// Work: the strips' rows (strip after strip) are cut into equal runs, one per
+// CTA; a run is cut at the strips' ends, or in half, into pieces.  Passes (pairs
+// of layers) follow one another in one cooperative launch: before a CTA loads
+// eight rows of its input in pass k it waits for those rows' flags of pass k - 1
+// in its strip and the two beside it.  That also orders the reuse of the
+// two alternating buffers: the readers in pass k - 1 of what row y of pass k
+// overwrites are the owners of rows y-2 .. y+2 of these strips, and pass k's row y
+// waited for all of them.  Even passes take a CTA's pieces in order, odd passes
+// in reverse, so a pass starts with the piece whose neighbours finished a
+// piece's time ago and its first loads do not wait.
+// Each layer has an MMA issuer and eight epilogue warps of its own (rows taken in
+// turn by two sets of four, one warp per TMEM lane quarter), so B's rows of one pass
+// never wait for A's rows of the next: every pass ends, whatever the others wait
+// for, and each wait is bounded all the same.
+constexpr int kChOutW = kTW - 2;      // output columns of a strip
+constexpr int kChIn = 10, kChMid = 8; // rows of the input (even) and of the middle ring
+constexpr int kChAcc = 8;             // row accumulators per layer
+constexpr int kChPub = 16;            // groups of stored rows between the epilogue and the publisher
+constexpr int kChMinH = 8;            // fewest rows of an image (the rings' phases, see the issuers)
+constexpr int kChMaxPass = 16;
+// producer, issuer of A, issuer of B, publisher of B's rows, 8 epilogue warps of A, 8 of B
+constexpr int kChThreads = 32 * (4 + 16);
+
+struct ChainArgs {
+  int B, H, W, strips;
+  int passes, c8_first;             // c8_first: channel chunks of the first layer's input (2 or 4)
+  const __nv_bfloat16* in;          // [B][H][c8_first][W][8]
+  __nv_bfloat16* mid[kChMaxPass];   // layer A's output of each pass, or NULL
+  __nv_bfloat16* out[kChMaxPass];   // layer B's output
+  const __nv_bfloat16* wpack[2 * kChMaxPass];
+  const float* bias[2 * kChMaxPass];
+  int* flags;                       // [passes][B][strips][H]
+  int epoch;
+  float alpha;
+  int* err;
+};
+
+struct ChainGeom {
+  static constexpr uint32_t P = kBoxW * 16;      // chunk plane stride
+  static constexpr uint32_t RS = 4 * P;          // ring row stride
+  static constexpr uint32_t WB = 9 * 4 * kCout * 16;
+  static constexpr uint32_t OFF_MID = kChIn * RS;
+  static constexpr uint32_t OFF_W = OFF_MID + kChMid * RS;
+  static constexpr uint32_t OFF_BIAS = OFF_W + 4 * WB;  // weights of two passes
+  static constexpr uint32_t OFF_BAR = OFF_BIAS + 2 * kChMaxPass * kCout * 4;
+  static constexpr uint32_t SMEM = OFF_BAR + 80 * 8 + 16 + 1024;
+  static_assert(SMEM <= 232448, "shared memory");
+};
+
+// A piece of a run: rows [y0, y1) of strip s of image b.
+struct ChainPiece { int b, s, y0, y1; };
+
+// The pieces of one CTA's run in the order of a pass.
+struct ChainRun {
+  long long lo, hi;
+  int H, strips, n;
+  bool halves;
+  __device__ __forceinline__ ChainRun(const ChainArgs& a) {
+    const long long total = (long long)a.B * a.strips * a.H;
+    lo = total * blockIdx.x / gridDim.x;
+    hi = total * (blockIdx.x + 1) / gridDim.x;
+    H = a.H;
+    strips = a.strips;
+    n = hi > lo ? (int)((hi - 1) / H - lo / H) + 1 : 0;
+    halves = n == 1 && hi - lo >= 16;
+    if (halves) n = 2;
+  }
+  __device__ __forceinline__ ChainPiece piece(int pass, int k) const {
+    if (pass & 1) k = n - 1 - k;
+    long long u = lo, v = hi;
+    if (halves) {
+      const long long m = (lo + hi) >> 1;
+      (k ? u : v) = m;
+    } else {
+      const long long c = lo / H + k;
+      if (c * H > u) u = c * H;
+      if ((c + 1) * H < v) v = (c + 1) * H;
+    }
+    ChainPiece p;
+    const int c = (int)(u / H);
+    p.b = c / strips;
+    p.s = c - p.b * strips;
+    p.y0 = (int)(u - (long long)c * H);
+    p.y1 = (int)(v - (long long)c * H);
+    return p;
+  }
+};
+
+// One input row added into the accumulators of the output rows whose kernel rows
+// dlo .. dhi it is: kernel row dy at ring block (b0 + dy) mod 8 of `tset`.  (The
+// epilogue leaves an accumulator it has read at zero, so every MMA accumulates.)
+template <int C8>
+__device__ __forceinline__ void chain_issue(uint32_t in_lo, uint32_t w_lo, uint32_t tset, int b0, int dlo, int dhi) {
+  constexpr uint32_t hi = tc::desc_hi(128);
+  constexpr uint32_t id96 = tc::make_idesc_bf16(128, 3 * kCout, false, false);
+  if (dlo == 0 && dhi == 2 && b0 <= kChAcc - 3) {
+    const uint32_t d0 = tset + (uint32_t)(b0 * kCout);
+#pragma unroll
+    for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+      for (int ks = 0; ks < C8 / 2; ++ks)
+        tc::mma_bf16(d0, tc::desc_join(in_lo + ((dx * 16 + ks * 2 * ChainGeom::P) >> 4), hi),
+                     tc::desc_join(w_lo + (dx * C8 + ks * 2) * kWRowsN, hi), id96, 1u);
+  } else {
+    // the window wraps around the ring, or lacks a kernel row at a piece's first or last rows
+    const int cut = min(dhi, kChAcc - 1 - b0);  // last kernel row before the wrap
+    const int n1 = cut - dlo + 1, e2 = max(cut + 1, dlo), n2 = dhi - e2 + 1;
+    const uint32_t c1 = tset + (uint32_t)(((b0 + dlo) & (kChAcc - 1)) * kCout);
+    const uint32_t c2 = tset + (uint32_t)(((b0 + e2) & (kChAcc - 1)) * kCout);
+    const uint32_t i1 = (id96 & ~(63u << 17)) | ((uint32_t)(n1 * (kCout / 8)) << 17);
+    const uint32_t i2 = (id96 & ~(63u << 17)) | ((uint32_t)(n2 * (kCout / 8)) << 17);
+#pragma unroll
+    for (int dx = 0; dx < 3; ++dx)
+#pragma unroll
+      for (int ks = 0; ks < C8 / 2; ++ks) {
+        const uint64_t ad = tc::desc_join(in_lo + ((dx * 16 + ks * 2 * ChainGeom::P) >> 4), hi);
+        const uint32_t bl = w_lo + (dx * C8 + ks * 2) * kWRowsN;
+        if (n1 > 0) tc::mma_bf16(c1, ad, tc::desc_join(bl + dlo * kCout, hi), i1, 1u);
+        if (n2 > 0) tc::mma_bf16(c2, ad, tc::desc_join(bl + e2 * kCout, hi), i2, 1u);
+      }
+  }
+}
+
+// One lane's pixel of a finished accumulator row: bias, LeakyReLU, bf16 (four 8-channel chunks).
+// MAX: 0 < alpha <= 1, for which max(z, alpha z) is LeakyReLU's value, bit for bit.
+template <bool MAX>
+__device__ __forceinline__ void chain_act(const uint32_t (&v)[32], const float4* bias, float alpha, uint4 (&o)[4]) {
+  const float2 al = make_float2(alpha, alpha);
+#pragma unroll
+  for (int ch = 0; ch < 4; ++ch) {
+    const float4 b0 = bias[2 * ch], b1 = bias[2 * ch + 1];
+    const float2 bb[4] = {{b0.x, b0.y}, {b0.z, b0.w}, {b1.x, b1.y}, {b1.z, b1.w}};
+    uint32_t w[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float2 z = __fadd2_rn(make_float2(__uint_as_float(v[ch * 8 + 2 * e]), __uint_as_float(v[ch * 8 + 2 * e + 1])),
+                                  bb[e]);
+      const float2 y = __fmul2_rn(z, al);
+      w[e] = MAX ? pack_bf16x2(fmaxf(z.x, y.x), fmaxf(z.y, y.y))
+                 : pack_bf16x2(z.x > 0.f ? z.x : y.x, z.y > 0.f ? z.y : y.y);
+    }
+    o[ch] = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+}
+
+__global__ void __launch_bounds__(kChThreads, 1) conv3x3_chain_kernel(const ChainArgs a) {
+  using G = ChainGeom;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* smem = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  uint64_t* in_full = reinterpret_cast<uint64_t*>(smem + G::OFF_BAR);  // [kChIn / 2] two input rows landed
+  uint64_t* a_done = in_full + kChIn;    // [kChIn] A's MMAs of the row completed: slot free, A's row i - 2 finished
+  uint64_t* mid_full = a_done + kChIn;   // [kChMid] middle row written
+  uint64_t* b_done = mid_full + kChMid;  // [kChMid] B's MMAs of the row completed
+  uint64_t* a_free = b_done + kChMid;    // [kChAcc] accumulator read
+  uint64_t* b_free = a_free + kChAcc;    // [kChAcc]
+  uint64_t* w_full = b_free + kChAcc;    // [4] a layer's weights landed
+  uint64_t* w_done = w_full + 4;         // [4] the layer's last MMA completed
+  uint64_t* stored = w_done + 4;         // [kChPub] a group of B's rows stored by its eight warps
+  static_assert(2 * kChIn + 2 * kChMid + 2 * kChAcc + 8 + kChPub <= 80, "barrier slots");
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + G::OFF_BAR + 80 * 8);
+  volatile int* gave_up = reinterpret_cast<volatile int*>(smem + G::OFF_BAR + 80 * 8 + 4);
+  volatile uint32_t* published = reinterpret_cast<volatile uint32_t*>(smem + G::OFF_BAR + 80 * 8 + 8);  // groups so far
+  float* sbias = reinterpret_cast<float*>(smem + G::OFF_BIAS);  // [layer][32]
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+
+  grid_dep_wait();
+  if (threadIdx.x == 0) {
+    *gave_up = 0;
+    for (int i = 0; i < kChIn; ++i) { tc::mbar_init(&in_full[i], 1); tc::mbar_init(&a_done[i], 1); }
+    for (int i = 0; i < kChMid; ++i) { tc::mbar_init(&mid_full[i], 4); tc::mbar_init(&b_done[i], 1); }
+    for (int i = 0; i < kChAcc; ++i) { tc::mbar_init(&a_free[i], 4); tc::mbar_init(&b_free[i], 4); }
+    for (int i = 0; i < 4; ++i) { tc::mbar_init(&w_full[i], 1); tc::mbar_init(&w_done[i], 1); }
+    for (int i = 0; i < kChPub; ++i) tc::mbar_init(&stored[i], 8);
+    *published = 0;
+    tc::fence_mbar_init();
+  }
+  for (int l = warp; l < 2 * a.passes; l += kChThreads / 32) sbias[l * kCout + lane] = a.bias[l][lane];
+  if (warp == 0) {
+    tc::tmem_alloc(tmem_slot, 512);
+    tc::tmem_relinquish();
+  }
+  tc::tc_fence_before();
+  __syncthreads();
+  tc::tc_fence_after();
+  const uint32_t tmem = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  if (warp >= 4 && warp < 8) {  // every accumulator starts at zero
+    for (int c = 0; c < 512; c += 32) tc::tmem_zero32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + c);
+    tc::tmem_wait_st();
+    tc::tc_fence_before();
+  }
+  __syncthreads();
+  tc::tc_fence_after();
+  const uint32_t sbase = tc::smem_u32(smem);
+  const ChainRun run(a);
+  // one thread's bounded wait; it also ends when another warp of the CTA gave up
+  auto wait1 = [&](uint64_t* bar, uint32_t parity, int code) {
+    if (tc::mbar_try_wait(bar, parity)) return true;
+    for (uint32_t n = 0; n < (1u << 22) && !*gave_up; ++n)
+      if (tc::mbar_try_wait(bar, parity)) return true;
+    if (!*gave_up) set_err(a.err, code);
+    *gave_up = 1;
+    return false;
+  };
+  // the same for a whole warp, with one result
+  auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
+    return (bool)__all_sync(0xffffffffu, wait1(bar, parity, code));
+  };
+
+  if (warp == 0) {
+    // ---------------- producer: two rows at a time ----------------
+    int slot = 0;
+    uint32_t ph = 0;  // phase of the ring's slots
+    bool ok = true;
+    for (int k = 0; k < a.passes && ok; ++k) {
+      const int c8 = k == 0 ? a.c8_first : 4;
+      const __nv_bfloat16* src = k == 0 ? a.in : a.out[k - 1];
+      // the two layers' weights (their buffers' last users are the layers of pass k - 2)
+      for (int l = 2 * k; l < 2 * k + 2; ++l) {
+        const int wb = l & 3;
+        if (!(ok = wait(&w_done[wb], ((l >> 2) & 1) ^ 1, 41))) break;
+        const uint32_t bytes = l == 0 ? (uint32_t)(9 * a.c8_first * kCout * 16) : G::WB;
+        if (lane == 0) {
+          tc::mbar_expect_tx(&w_full[wb], bytes);
+          tc::bulk_load(smem + G::OFF_W + wb * G::WB, a.wpack[l], bytes, &w_full[wb]);
+        }
+        __syncwarp();
+      }
+      for (int q = 0; q < run.n && ok; ++q) {
+        const ChainPiece p = run.piece(k, q);
+        const int gx0 = p.s * kChOutW - 2, xa = max(gx0, 0), xb = min(gx0 + kBoxW, a.W);
+        const int left = xa - gx0, right = xb < gx0 + kBoxW ? xb - gx0 : -1;  // pixels to clear on each side
+        const uint32_t bytes = (uint32_t)(xb - xa) * 16;
+        const int rr = lane >= c8 ? 1 : 0, ch = lane - rr * c8;  // this lane's row of the two, and its chunk
+        const __nv_bfloat16* row = src + (((size_t)p.b * a.H * c8 + ch) * a.W + xa) * 8;
+        const int first = p.y0 - 2, end = p.y1 + 2;
+        // the flags of eight rows of the previous pass in this strip and its neighbours: lane -> (row, strip)
+        const int fs = p.s + lane % 3 - 1, fr = lane / 3;
+        const int* flag = a.flags + (((size_t)(k - 1) * a.B + p.b) * a.strips + fs) * a.H;
+        auto flag_of = [&](int y) { return k > 0 && lane < 24 && fs >= 0 && fs < a.strips && y >= 0 && y < a.H && y < end; };
+        int seen = flag_of(first + fr) ? tc::ld_relaxed_gpu(flag + first + fr) : a.epoch;
+        for (int y = first; y < end; y += 2) {
+          if (k > 0 && ((y - first) & 7) == 0) {
+            const int yy = y + fr;
+            uint32_t n = 0;
+            while (seen != a.epoch && ++n < (1u << 22) && !*gave_up) {
+              __nanosleep(20);
+              seen = tc::ld_relaxed_gpu(flag + yy);
+            }
+            if (!__all_sync(0xffffffffu, seen == a.epoch)) {
+              if (lane == 0 && !*gave_up) set_err(a.err, 42);
+              *gave_up = 1;
+              ok = false;
+              break;
+            }
+            tc::fence_acq_rel_gpu();         // the eight rows' stores are visible to this warp,
+            tc::fence_proxy_async_global();  // and to its bulk copies
+            // the next eight rows' flags, looked at when they are due
+            seen = flag_of(yy + 8) ? tc::ld_relaxed_gpu(flag + yy + 8) : a.epoch;
+          }
+          const bool two = y + 1 < end;
+          // A's rows are multiplied in order: the second slot's release covers the first's
+          if (!(ok = wait(&a_done[slot + (two ? 1 : 0)], ph ^ 1, 43))) break;
+          const bool live0 = y >= 0 && y < a.H, live1 = two && y + 1 >= 0 && y + 1 < a.H;
+          unsigned char* dst = smem + slot * G::RS;
+          if (!live0 || (two && !live1) || (y < first + kChIn && (left > 0 || right >= 0))) {
+            // rows outside the domain; beside it two pixels on the left and the one past the right
+            // border that an output reads (the copies leave them alone: once per slot and piece)
+            const uint4 z = make_uint4(0, 0, 0, 0);
+            for (int r = 0; r < (two ? 2 : 1); ++r) {
+              unsigned char* d = dst + r * G::RS;
+              if (!(r ? live1 : live0)) {
+                for (int i = lane; i < c8 * kBoxW; i += 32) reinterpret_cast<uint4*>(d)[i] = z;
+              } else if (lane < 3 * c8) {
+                const int i = lane / c8;
+                uint4* plane = reinterpret_cast<uint4*>(d + (lane - i * c8) * G::P);
+                if (i < 2 ? i < left : right >= 0) plane[i < 2 ? i : right] = z;
+              }
+            }
+            tc::fence_proxy_async_smem();
+            __syncwarp();
+          }
+          if (lane == 0) tc::mbar_expect_tx(&in_full[slot >> 1], (uint32_t)c8 * bytes * ((live0 ? 1 : 0) + (live1 ? 1 : 0)));
+          __syncwarp();
+          if (lane < 2 * c8 && (rr ? live1 : live0))
+            tc::bulk_load(dst + rr * G::RS + ch * G::P + left * 16, row + (size_t)(y + rr) * c8 * a.W * 8, bytes,
+                          &in_full[slot >> 1]);
+          slot += 2;
+          if (slot == kChIn) {
+            slot = 0;
+            ph ^= 1;
+          }
+        }
+      }
+    }
+  } else if (warp <= 2) {
+    // ---------------- MMA issuers: warp 1 layer A, warp 2 layer B, one thread each ----------------
+    if (tc::elect_one()) {
+      const bool layer_a = warp == 1;
+      const int ring = layer_a ? kChIn : kChMid;
+      uint64_t *full = layer_a ? in_full : mid_full, *done = layer_a ? a_done : b_done,
+               *freed = layer_a ? a_free : b_free;
+      const uint32_t rbase = sbase + (layer_a ? 0u : G::OFF_MID);
+      const uint32_t tset = tmem + (layer_a ? 0u : (uint32_t)(kChAcc * kCout));
+      int slot = 0;
+      uint32_t ph = 0, o = 0;  // ring slot and phase; the output row the next input row starts
+      bool ok = true;
+      for (int k = 0; k < a.passes && ok; ++k) {
+        const int l = 2 * k + (layer_a ? 0 : 1);
+        const uint32_t w_lo = tc::desc_lo(sbase + G::OFF_W + (l & 3) * G::WB, kWRowsN * 16);
+        const bool narrow = l == 0 && a.c8_first == 2;
+        if (!(ok = wait1(&w_full[l & 3], (l >> 2) & 1, 44))) break;
+        for (int q = 0; q < run.n && ok; ++q) {
+          const ChainPiece p = run.piece(k, q);
+          const int rows = p.y1 - p.y0 + (layer_a ? 2 : 0);  // output rows of this layer
+          for (int i = 0; i < rows + 2; ++i) {
+            // input row i starts output row i and finishes output row i - 2
+            if (!layer_a || !(i & 1))
+              if (!(ok = wait1(layer_a ? &full[slot >> 1] : &full[slot], ph, 45))) break;
+            // (Also where the row starts none: it keeps this warp from lapping an epilogue warp that
+            // still waits for an earlier phase of done[slot].  Rows of a layer's input and output
+            // differ by two per piece; with pieces in the middle of a run at least kChMinH high, the
+            // next phase of a ring slot always lies behind the release of the row waited for.)
+            const uint32_t blk = o & (kChAcc - 1);
+            if (!(ok = wait1(&freed[blk], ((o / kChAcc) & 1) ^ 1, 46))) break;
+            tc::tc_fence_after();
+            const uint32_t in_lo = tc::desc_lo(rbase + slot * G::RS, G::P);
+            const int b0 = kChAcc - 1 - (int)blk, dlo = i >= rows ? i - rows + 1 : 0, dhi = min(i, 2);
+            if (narrow)
+              chain_issue<2>(in_lo, w_lo, tset, b0, dlo, dhi);
+            else
+              chain_issue<4>(in_lo, w_lo, tset, b0, dlo, dhi);
+            tc::mma_commit(&done[slot]);
+            ++o;
+            if (++slot == ring) {
+              slot = 0;
+              ph ^= 1;
+            }
+          }
+          o -= 2;  // the last two input rows start none
+          if (layer_a && (slot & 1)) {  // rows arrive in pairs: the last one was alone
+            tc::mma_commit(&done[slot]);
+            if (++slot == ring) {
+              slot = 0;
+              ph ^= 1;
+            }
+          }
+        }
+        if (ok) tc::mma_commit(&w_done[l & 3]);
+      }
+    }
+    __syncwarp();
+  } else if (warp == 3) {
+    // ---------------- publisher: B's rows, four at a time, once their eight warps stored them ----------------
+    uint32_t g = 0;
+    bool ok = true;
+    for (int k = 0; k < a.passes && ok; ++k)
+      for (int q = 0; q < run.n && ok; ++q) {
+        const ChainPiece p = run.piece(k, q);
+        int* f = a.flags + (((size_t)k * a.B + p.b) * a.strips + p.s) * a.H;
+        for (int y = p.y0; y < p.y1; y += 4) {
+          if (!(ok = wait(&stored[g % kChPub], (g / kChPub) & 1, 48))) break;
+          if (lane < 4 && y + lane < p.y1) tc::st_release_gpu(f + y + lane, a.epoch);
+          __syncwarp();
+          if (lane == 0) *published = ++g; else ++g;
+        }
+      }
+  } else {
+    // ---------------- epilogues: warps 4-11 layer A, warps 12-19 layer B ----------------
+    const bool layer_a = warp < 12;
+    const uint32_t set = (warp >> 2) & 1;  // takes the even or the odd rows
+    const int q4 = warp & 3;               // TMEM lane quarter
+    const int px = q4 * 32 + lane;         // pixel of the row = TMEM lane
+    const uint32_t tset = tmem + ((uint32_t)(q4 * 32) << 16) + (layer_a ? 0u : (uint32_t)(kChAcc * kCout));
+    uint64_t *done = layer_a ? a_done : b_done, *freed = layer_a ? a_free : b_free;
+    const uint32_t ring = layer_a ? kChIn : kChMid;
+    const bool leaky_max = a.alpha > 0.f && a.alpha <= 1.f;
+    uint32_t o = 0;   // finished rows of this layer so far
+    uint32_t in = 0;  // rows of this layer's input before the piece
+    uint32_t g = 0;   // groups of B's rows so far
+    bool ok = true;
+    for (int k = 0; k < a.passes && ok; ++k) {
+      const float4* bias = reinterpret_cast<const float4*>(sbias + (2 * k + (layer_a ? 0 : 1)) * kCout);
+      __nv_bfloat16* dst = layer_a ? a.mid[k] : a.out[k];
+      for (int q = 0; q < run.n && ok; ++q) {
+        const ChainPiece p = run.piece(k, q);
+        const int nb = p.y1 - p.y0, rows = layer_a ? nb + 2 : nb;
+        const int y0 = layer_a ? p.y0 - 1 : p.y0;               // first row
+        const int x = p.s * kChOutW + (layer_a ? px - 1 : px);  // this lane's column
+        const bool col = x >= 0 && x < a.W;
+        // stored by this strip
+        const bool mine = dst != nullptr && col && (layer_a ? px >= 1 && px <= kChOutW : px < kChOutW);
+        for (int j = 0; j < rows; ++j, ++o) {
+          if ((o & 1) == set) {
+            // row j is complete with its input row j + 2
+            const uint32_t r = in + j + 2;
+            if (!(ok = wait(&done[r % ring], (r / ring) & 1, 47))) break;
+            tc::tc_fence_after();
+            uint32_t v[32];
+            const uint32_t acc = tset + (uint32_t)((kChAcc - 1 - (int)(o % kChAcc)) * kCout);
+            tc::tmem_ld32(acc, v);
+            tc::tmem_wait_ld();
+            tc::tmem_zero32(acc);
+            tc::tmem_wait_st();
+            tc::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) tc::mbar_arrive(&freed[o % kChAcc]);
+            uint4 w[4];
+            if (leaky_max)
+              chain_act<true>(v, bias, a.alpha, w);
+            else
+              chain_act<false>(v, bias, a.alpha, w);
+            const int y = y0 + j;
+            if (layer_a) {
+              if (!col || y < 0 || y >= a.H) {
+#pragma unroll
+                for (int ch = 0; ch < 4; ++ch) w[ch] = make_uint4(0, 0, 0, 0);
+              }
+              // into the middle ring once B has read the row that lies there
+              if (!(ok = wait(&b_done[o % kChMid], ((o / kChMid) & 1) ^ 1, 49))) break;
+              unsigned char* m = smem + G::OFF_MID + (o % kChMid) * G::RS + px * 16;
+#pragma unroll
+              for (int ch = 0; ch < 4; ++ch) *reinterpret_cast<uint4*>(m + ch * G::P) = w[ch];
+              tc::fence_proxy_async_smem();
+              __syncwarp();
+              if (lane == 0) tc::mbar_arrive(&mid_full[o % kChMid]);
+            }
+            if (mine && y >= p.y0 && y < p.y1) {
+              uint4* g = reinterpret_cast<uint4*>(dst) + (((size_t)p.b * a.H + y) * 4) * a.W + x;
+#pragma unroll
+              for (int ch = 0; ch < 4; ++ch) g[(size_t)ch * a.W] = w[ch];
+            }
+          }
+          if (!layer_a && ((j & 3) == 3 || j == rows - 1)) {
+            // a group of rows is stored: the publisher's turn when all eight warps say so
+            tc::fence_proxy_async_global();
+            __syncwarp();
+            for (uint32_t n = 0; g >= *published + kChPub && n < (1u << 22) && !*gave_up; ++n) __nanosleep(20);
+            if (lane == 0) tc::mbar_arrive(&stored[g % kChPub]);
+            ++g;
+          }
+        }
+        in += layer_a ? (uint32_t)((nb + 5) & ~1) : (uint32_t)(nb + 2);  // A's input ring advances in pairs
+      }
+    }
+  }
+  __syncthreads();
+  if (*gave_up)  // let the copies and MMAs in flight end
+    for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+  if (warp == 0) {
+    tc::tc_fence_after();
+    tc::tmem_dealloc(tmem, 512);
+  }
+}
+
+// ---------------------------------------------------------------------------
 // weight gradient
 // ---------------------------------------------------------------------------
 struct WgradArgs {
@@ -1398,6 +1874,79 @@ extern "C" size_t igm_conv3x3_stack_flags_len(int batch, int height, int width, 
   if (batch < 1 || height < 1 || width < 1) return 0;
   const int r = stack_rows(batch, height, width);
   return (size_t)nlayers * batch * ((width + kTW - 1) / kTW) * ((height + r - 1) / r);
+}
+
+extern "C" int igm_conv3x3_chain(int batch, int height, int width, int nlayers, int cin_first, const void* x,
+                                 void* const* mids, void* const* outs, const void* const* wpacks,
+                                 const float* const* biases, int* flags, int epoch, float alpha, int* err,
+                                 void* stream) {
+  using G = ChainGeom;
+  IGM_CHECK_ARG(batch >= 1 && height >= kChMinH && width >= 1 && batch <= 65535, IGM_ERR_BAD_SHAPE,
+                "igm_conv3x3_chain: bad shape %dx%dx%d (height >= %d)", batch, height, width, kChMinH);
+  IGM_CHECK_ARG(nlayers >= 2 && nlayers % 2 == 0 && nlayers <= 2 * kChMaxPass, IGM_ERR_BAD_SHAPE,
+                "igm_conv3x3_chain: an even number of layers, 2 .. %d", 2 * kChMaxPass);
+  IGM_CHECK_ARG(cin_first == 16 || cin_first == 32, IGM_ERR_UNSUPPORTED, "igm_conv3x3_chain: cin_first must be 16 or 32");
+  IGM_CHECK_ARG(x && mids && outs && wpacks && biases && flags && epoch != 0, IGM_ERR_BAD_ARGUMENT,
+                "igm_conv3x3_chain: NULL argument or zero epoch");
+  IGM_CHECK_ARG(((uintptr_t)x & 15) == 0, IGM_ERR_BAD_ARGUMENT, "igm_conv3x3_chain: activations must be 16-byte aligned");
+  ChainArgs a{};
+  a.B = batch; a.H = height; a.W = width;
+  a.strips = (width + kChOutW - 1) / kChOutW;
+  a.passes = nlayers / 2;
+  a.c8_first = cin_first / 8;
+  a.in = (const __nv_bfloat16*)x;
+  for (int k = 0; k < a.passes; ++k) {
+    IGM_CHECK_ARG(outs[k] && ((uintptr_t)outs[k] & 15) == 0 && ((uintptr_t)mids[k] & 15) == 0, IGM_ERR_BAD_ARGUMENT,
+                  "igm_conv3x3_chain: pass %d: NULL or unaligned output", k);
+    IGM_CHECK_ARG(outs[k] != (k ? outs[k - 1] : x) && (!mids[k] || (mids[k] != outs[k] && mids[k] != (k ? outs[k - 1] : x))),
+                  IGM_ERR_BAD_ARGUMENT, "igm_conv3x3_chain: pass %d: an output aliases the pass's input or other output", k);
+    a.mid[k] = (__nv_bfloat16*)mids[k];
+    a.out[k] = (__nv_bfloat16*)outs[k];
+  }
+  for (int l = 0; l < nlayers; ++l) {
+    IGM_CHECK_ARG(wpacks[l] && biases[l] && ((uintptr_t)wpacks[l] & 15) == 0, IGM_ERR_BAD_ARGUMENT,
+                  "igm_conv3x3_chain: layer %d: NULL or unaligned pointer", l);
+    a.wpack[l] = (const __nv_bfloat16*)wpacks[l];
+    a.bias[l] = biases[l];
+  }
+  a.flags = flags;
+  a.epoch = epoch;
+  a.alpha = alpha;
+  a.err = err;
+  static bool configured = false;
+  int rc = set_smem(conv3x3_chain_kernel, G::SMEM, &configured);
+  if (rc) return rc;
+  const long long rows = (long long)batch * a.strips * height;
+  const int grid = (int)(rows < sm_count() ? rows : sm_count());
+  // cooperative: every CTA resident at once, which the row flags rely on
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(kChThreads);
+  cfg.dynamicSmemBytes = G::SMEM;
+  cfg.stream = as_stream(stream);
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeCooperative;
+  attr[0].val.cooperative = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, conv3x3_chain_kernel, a);
+  return launch_status("conv3x3_chain_kernel");
+}
+
+extern "C" size_t igm_conv3x3_chain_flags_len(int batch, int height, int width, int nlayers) {
+  if (batch < 1 || height < kChMinH || width < 1 || nlayers < 2) return 0;
+  return (size_t)(nlayers / 2) * batch * ((width + kChOutW - 1) / kChOutW) * height;
+}
+
+// A pass of the chain reads two halo rows above and below each piece of a run of rows and takes 8 us from
+// the last pass's flags to its own, so it pays with long runs.  16 layers, stack and first layer against
+// the chain, us: 20 rows per SM (500 x 750) 159 / 181, 27 (2 x 500 x 500) 192 / 207, 38 (700 x 1003) 255 / 251, 54
+// (1000 x 1000) 362 / 324, 235 (2048 x 2048) 1535 / 1229, 913 (4096 x 4096) 6190 / 5390.  With every activation kept it
+// saves reads only; the whole network's forward then takes, stack / chain: 54 rows 428 / 438, 108 (8 x 500 x 500)
+// 911 / 806, 235 1915 / 1732.
+extern "C" int igm_conv3x3_chain_pays(int batch, int height, int width, int keep_all) {
+  return batch >= 1 && height >= kChMinH && width >= 1 &&
+         (long long)batch * ((width + kChOutW - 1) / kChOutW) * height >= (keep_all ? 80LL : 45LL) * sm_count();
 }
 
 extern "C" int igm_conv1x1_wgrad(int batch, int height, int width, const void* x, const void* g, float* partials,

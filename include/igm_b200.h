@@ -544,6 +544,22 @@ IGM_API int igm_conv3x3_stack(int batch, int height, int width, int nlayers, con
                               const void* const* wpacks, const float* const* biases, int* flags, int epoch,
                               float alpha, int* err, void* stream);
 IGM_API size_t igm_conv3x3_stack_flags_len(int batch, int height, int width, int nlayers);
+
+/* A chain of nlayers (even) forward layers, two per pass over memory: layer 0
+ * has cin_first (16 or 32) input channels, the others 32; weights and biases as
+ * igm_conv3x3's forward mode.  Pass k computes layers 2k and 2k + 1: outs[k]
+ * gets layer 2k + 1's output, mids[k] (may be NULL) layer 2k's.  outs may
+ * alternate between two buffers, neither of them x.  flags: device int buffer of
+ * igm_conv3x3_chain_flags_len ints holding no value equal to epoch (non-zero); the call
+ * leaves it filled with epoch.  height >= 8.  The same bits as nlayers igm_conv3x3 calls; for
+ * grids that give every SM some rows (the caller's choice). */
+IGM_API int igm_conv3x3_chain(int batch, int height, int width, int nlayers, int cin_first, const void* x,
+                              void* const* mids, void* const* outs, const void* const* wpacks,
+                              const float* const* biases, int* flags, int epoch, float alpha, int* err, void* stream);
+IGM_API size_t igm_conv3x3_chain_flags_len(int batch, int height, int width, int nlayers);
+/* 1 where the chain is faster than igm_conv3x3 and igm_conv3x3_stack, else 0
+ * (keep_all: with every layer's output stored, mids given). */
+IGM_API int igm_conv3x3_chain_pays(int batch, int height, int width, int keep_all);
 /* Both gradients of a 32 -> 32 channel layer in one pass over its inputs
  * (replaces igm_conv3x3(IGM_CONV_DGRAD) + igm_conv3x3_wgrad for the hidden
  * layers; the Keras GradientTape of emulate.py:252 through Conv2D(3x3) +

@@ -11,6 +11,7 @@ import numpy as np
 import pytest
 import torch
 
+from igm_b200 import _lib as L
 from igm_b200 import kernels as K
 from igm_b200.cnn import CNN
 from igm_b200.emulator import EmulatorOptimizer, train_step
@@ -229,3 +230,29 @@ def test_production_network_forward_and_gradient_match_oracle():
         worst = max(worst, e)
         assert e < 1e-1, (i, s, e)
     print(f"16-layer parameter gradients: worst relative L2 {worst:.2e}")
+
+
+@pytest.mark.parametrize("nl", [2, 5])
+@pytest.mark.parametrize("keep", [False, True])
+def test_two_layers_per_pass_gives_the_same_bits(nl, keep):
+    """The network on a domain large enough for igm_conv3x3_chain (an odd last
+    layer by itself) against the same network layer by layer: velocities and
+    kept activations bit for bit."""
+    h, w, nz = (1703 if keep else 1003), 999, 3
+    net = CNN(nb_layers=nl, cin=5, nout=2 * nz, init="he_normal", seed=3, scales=[1 / 300, 1 / 3000, 0.01, 10, 0.01])
+    g = torch.Generator().manual_seed(1)
+    f = [(torch.rand(h, w, generator=g) * s).cuda() for s in (300.0, 3000.0, 100.0, 0.1)]
+    buf = net.buffers(1, h, w, train=keep)
+    assert buf["chain"]
+    net.prepare_input(f, 50.0, [(0, 0)], h, w, buf)
+    U, V = (t.clone() for t in net.forward(buf, 1, h, w, keep_acts=keep))
+    acts = [a.clone() for a in buf["acts"]] if keep else None
+    flags = buf["flags"]
+    buf["chain"] = False
+    buf["flags"] = torch.zeros(int(L.lib().igm_conv3x3_stack_flags_len(1, h, w, nl - 1)), dtype=torch.int32, device="cuda")
+    U2, V2 = net.forward(buf, 1, h, w, keep_acts=keep)
+    net.check_errors()
+    assert torch.equal(U, U2) and torch.equal(V, V2)
+    if keep:
+        assert all(torch.equal(a, b) for a, b in zip(acts, buf["acts"]))
+    assert flags.numel() == (nl // 2) * 8 * h

@@ -310,3 +310,51 @@ def test_head_forward(B, H, W, nz, mask):
     assert float((got - y).abs().max()) <= 1e-5 * float(y.abs().max()) + 1e-6
     if mask:
         assert bool((got[(thk <= 0)[:, None].expand_as(got)] == 0).all())
+
+
+def _chain(lib, st, B, H, W, nl, cin, keep, x, ws, bs, flags, epoch, err):
+    """igm_conv3x3_chain on x: (outputs of every layer or None, last output)."""
+    P = __import__("ctypes").c_void_p
+    shape = (B, H, 4, W, 8)
+    n = nl // 2
+    two = [torch.full(shape, float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(2)]
+    outs = [torch.full(shape, float("nan"), dtype=torch.bfloat16, device="cuda") if keep else two[k % 2] for k in range(n)]
+    mids = [torch.full(shape, float("nan"), dtype=torch.bfloat16, device="cuda") if keep else None for _ in range(n)]
+    L.check(lib.igm_conv3x3_chain(B, H, W, nl, cin, x.data_ptr(), (P * n)(*[m.data_ptr() if keep else None for m in mids]),
+                                  (P * n)(*[o.data_ptr() for o in outs]), (P * nl)(*[w.data_ptr() for w in ws]),
+                                  (P * nl)(*[b.data_ptr() for b in bs]), flags.data_ptr(), epoch, 0.01, err.data_ptr(), st))
+    torch.cuda.synchronize()
+    assert int(err.item()) == 0
+    return [t for p in zip(mids, outs) for t in p] if keep else None, outs[-1]
+
+
+@pytest.mark.parametrize("B,H,W,nl,cin", [(1, 8, 1, 2, 32), (3, 8, 4000, 4, 16), (1, 37, 126, 2, 16), (1, 40, 127, 4, 16), (2, 11, 253, 4, 32),
+                                          (8, 64, 64, 6, 16), (1, 300, 125, 16, 16), (64, 33, 130, 4, 16),
+                                          (1, 1000, 1000, 16, 16), (1, 149, 400, 8, 32)])
+def test_conv_chain(B, H, W, nl, cin):
+    """igm_conv3x3_chain: two layers per pass, bit for bit what nl igm_conv3x3
+    calls write -- strips of 126 columns and runs of rows around their ends,
+    with every activation kept and with the outputs alternating between two
+    buffers, twice on one flag buffer."""
+    g = torch.Generator().manual_seed(B * 7 + H * 3 + W + nl)
+    lib, st = L.lib(), L.stream_ptr()
+    x = torch.randn(B, H, cin // 8, W, 8, generator=g).to(torch.bfloat16).cuda()
+    cs = [cin] + [32] * (nl - 1)
+    ws = [(torch.randn(9 * c * 32, generator=g) * (1.3 / np.sqrt(9 * c))).to(torch.bfloat16).cuda() for c in cs]
+    bs = [(torch.randn(32, generator=g) * 0.1).cuda() for _ in range(nl)]
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ref, cur = [], x
+    for k in range(nl):
+        y = torch.empty(B, H, 4, W, 8, dtype=torch.bfloat16, device="cuda")
+        L.check(lib.igm_conv3x3(0, B, H, W, cs[k], cur.data_ptr(), ws[k].data_ptr(), bs[k].data_ptr(), None,
+                                y.data_ptr(), None, 0, 0.01, err.data_ptr(), st))
+        ref.append(y)
+        cur = y
+    flags = torch.zeros(int(lib.igm_conv3x3_chain_flags_len(B, H, W, nl)), dtype=torch.int32, device="cuda")
+    for epoch, keep in ((1, True), (2, False), (3, False)):
+        acts, last = _chain(lib, st, B, H, W, nl, cin, keep, x, ws, bs, flags, epoch, err)
+        assert bool((flags == epoch).all())
+        assert torch.equal(last, ref[-1])
+        if keep:
+            for k in range(nl):
+                assert torch.equal(acts[k], ref[k]), k
