@@ -969,9 +969,17 @@ static int level_map(CUtensorMap* m, const void* base, const igm_grid* g, int pl
   cuuint64_t strides[2] = {(cuuint64_t)g->nx * sizeof(T), (cuuint64_t)g->ny * g->nx * sizeof(T)};
   cuuint32_t box[3] = {(cuuint32_t)Box<T>::BW, (cuuint32_t)(TYC + 1), 1};
   cuuint32_t es[3] = {1, 1, 1};
-  CUresult r = enc(m, sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3,
-                   const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encode = [&]() {
+    return enc(m, sizeof(T) == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 3,
+               const_cast<void*>(base), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+               CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  if (r == CUDA_ERROR_INVALID_CONTEXT) {
+    // a thread that has not called the runtime yet (autograd's, when its buffers come from a cache)
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = encode();
+  }
   if (r != CUDA_SUCCESS) {
     set_error("cuTensorMapEncodeTiled (level tiles) failed (CUresult %d)", (int)r);
     return IGM_ERR_CUDA;

@@ -216,3 +216,22 @@ def test_backward_scale_on_the_device(dtype, gout):
     dU, dV = torch.autograd.grad(iceflow_energy(U, V, *f, 100.0, dz), [U, V], grad_outputs=g)
     _, rU, rV = K.energy(U.detach(), V.detach(), *f, 100.0, dz, grad=True, grad_scale=float(g) / ((ny - 1) * (nx - 1)))
     assert torch.equal(dU, rU) and torch.equal(dV, rV)
+
+
+def test_a_thread_without_a_context():
+    """The energy from a thread that has made no CUDA runtime call of its own
+    (autograd's backward thread, with buffers from the caching allocator)."""
+    import threading
+    st = O.valley_glacier(33, 40, 100.0, seed=9)
+    f = [dev(st[k], torch.float32) for k in ["thk", "usurf", "arrhenius", "slidingco"]]
+    dz = O.compute_zeta_dzeta(O.compute_levels(4, 4.0))[1].numpy()
+    U = torch.ones((4, 33, 40), device="cuda")
+    ref = K.energy(U, U, *f, 100.0, dz, grad=True)
+    keep = [torch.empty_like(U) for _ in range(4)]
+    del keep  # freed blocks that the thread's allocations reuse
+    got = []
+    t = threading.Thread(target=lambda: got.append(K.energy(U, U, *f, 100.0, dz, grad=True, terms_out=torch.empty_like(ref[0]))))
+    t.start()
+    t.join()
+    torch.cuda.synchronize()
+    assert len(got) == 1 and all(torch.equal(a, b) for a, b in zip(got[0], ref))
