@@ -132,6 +132,7 @@ SIGNATURES = {
     "igm_cnn_layer1_forward": (I, [I, I, I, I, P, P, P, P, D, P, P, P, C.c_float, P, P]),
     "igm_cnn_layer1_wgrad": (I, [I, I, I, I, P, P, P, P, D, P, P, P, I, P]),
     "igm_cnn_head_forward": (I, [I, I, I, I, P, P, P, C.c_float, P, P, P, P]),
+    "igm_cnn_head_inference": (I, [I, I, I, I, P, P, P, C.c_float] + [P] * 12),
     "igm_cnn_head_partial_len": (C.c_size_t, [I]),
     "igm_cnn_head_backward": (I, [I, I, I, I, P, P, P, P, C.c_float, C.c_float, P, P, I, P]),
     "igm_reduce_partials": (I, [P, I, I, I, P, I, P]),

@@ -172,10 +172,12 @@ class CNN:
     def _scales(self):
         return (C.c_float * 5)(*[float(s) for s in self.scales])
 
-    def forward(self, buf, B, h, w, thk_mask=None, keep_acts=False):
+    def forward(self, buf, B, h, w, thk_mask=None, keep_acts=False, vert_weight=None):
         """Runs the network on the windowed fields of ``buf`` (prepare_input):
         the first layer on the split (x_h, x_l, x_h) input, the 3x3 layers, the
-        head -- all convolutions on the tensor cores; U, V into buf."""
+        head -- all convolutions on the tensor cores; U, V into buf.  With
+        ``vert_weight`` (needs nout <= 32) returns (U, V, derived), derived what
+        kernels.velocity_reduce(U, V, mask=False) returns, from the head's pass."""
         lib, st = L.lib(), L.stream_ptr()
         acts = buf["acts"]
         if buf["chain"]:
@@ -206,6 +208,19 @@ class CNN:
             x = ys[-1]
         hw = self.params.data_ptr() + 4 * self.offsets[2 * self.L]
         hb = self.params.data_ptr() + 4 * self.offsets[2 * self.L + 1]
+        if vert_weight is not None:
+            d = [torch.empty((B, h, w), dtype=torch.float32, device=self.device) for _ in range(6)]
+            d.append(torch.empty(1, dtype=torch.float32, device=self.device))
+            vw = (C.c_double * self.nz)(*np.asarray(vert_weight, dtype=np.float64).reshape(-1)[:self.nz].tolist())
+            rc = lib.igm_cnn_head_inference(B, h, w, self.nz, _p(x), hw, hb, self.out_scale, _p(buf["U"]), _p(buf["V"]),
+                                            _p(thk_mask), vw, *[_p(t) for t in d], st)
+            L.check(rc, "igm_cnn_head_inference")
+            return buf["U"], buf["V"], tuple(d)
+        if not keep_acts and self.nout <= 32:
+            rc = lib.igm_cnn_head_inference(B, h, w, self.nz, _p(x), hw, hb, self.out_scale, _p(buf["U"]), _p(buf["V"]),
+                                            _p(thk_mask), None, *[None] * 7, st)
+            L.check(rc, "igm_cnn_head_inference")
+            return buf["U"], buf["V"]
         rc = lib.igm_cnn_head_forward(B, h, w, self.nz, _p(x), hw, hb, self.out_scale, _p(buf["U"]), _p(buf["V"]),
                                       _p(thk_mask), st)
         L.check(rc, "igm_cnn_head_forward")

@@ -16,6 +16,7 @@
 
 #include "common.cuh"
 #include "reduce.cuh"
+#include "tc.cuh"
 
 namespace igm {
 
@@ -226,6 +227,231 @@ __global__ void __launch_bounds__(256) head_fwd_kernel(int B, int H, int W, int 
       const int k = j < nz ? j : j - nz;
       dst[(b * nz + k) * plane + rem] = sv;
     }
+  }
+}
+
+// Head of an inference, for up to 32 outputs: U and V and, where wanted, the derived velocities
+// (velbar, velbase, velsurf, the CFL maximum) that velocity_reduce_kernel would read
+// them again for, formed by the lane that holds the pixel's column, with that kernel's operations
+// in its order.  The products are on the tensor cores: activations are bf16 and an FP32 weight is
+// the exact sum of three bf16 parts, so they are exact; mma.sync m16n8k16 sums
+// them in FP32, the lowest parts first (the FMA chains above cost a weight load from shared
+// memory per two channels, 990 instructions per pixel).  The training's forward keeps
+// those: its trajectory is held to their rounding.  The weights live in registers as B fragments.
+// A warp takes 32 pixels of a row: their activations (4 planes of 512 B) arrive by bulk copies
+// in a ring of kHmStages of its own, whose planes ldmatrix reads as they lie, and the sums are
+// exchanged through shared memory so that a lane owns a pixel and whole lines of every output plane
+// are stored.  A pixel with a sum that is not finite is evaluated again in FP32 (a zero part times an
+// infinite activation is NaN).
+// Bound by its 64 B in and 8 Nz + 24 B out per pixel; FMA chains and velocity_reduce_kernel, and
+// now: 1000 x 1000 x 10 83 and 39.5 us (4.3 TB/s), 4096 x 4096 x 16 1652 and 756, 301 x 333 x 5
+// 13.5 and 10.6.  Error of U and V against 64 bits 1.1e-7 and now 6.9e-8 (2-norm).
+struct HeadDerived {
+  float w[kF / 2];  // vertical weights
+  float *ubar, *vbar, *ub0, *vb0, *us0, *vs0;
+  float* velomax;
+};
+
+__device__ __forceinline__ void mma_16816(float (&d)[4], const uint32_t (&a)[4], const uint32_t (&b)[2],
+                                          const float (&c)[4]) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, "
+      "{%10, %11, %12, %13};\n"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]), "f"(c[0]), "f"(c[1]), "f"(c[2]), "f"(c[3]));
+}
+
+// Four 8 x 8 b16 matrices, a row of 16 B per lane's address.
+__device__ __forceinline__ void ldmatrix_x4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+               : "r"(addr)
+               : "memory");
+}
+
+constexpr int kHmWarps = 8;
+constexpr int kHmStages = 4;
+template <int NT>
+struct HeadMmaSmem {
+  static constexpr int S = NT * 8 + 1;  // a pixel's row of sums: odd, so that 32 rows fall on 32 banks
+  unsigned char ring[kHmWarps][kHmStages][4 * 512];
+  float sums[kHmWarps][32 * S];
+  float bias[NT * 8];
+  float weight[NT * 8];  // the vertical weight of each output's level
+  uint64_t full[kHmWarps][kHmStages];
+};
+// One kernel per number of levels: which output belongs to which plane is then known at each step.
+template <int NZ>
+__global__ void __launch_bounds__(kHmWarps * 32, 2)
+    head_fwd_mma_kernel(int B, int H, int W, const __nv_bfloat16* act, const float* wh, const float* bh,
+                        float out_scale, float* U, float* V, const float* thk_mask, const HeadDerived dv) {
+  grid_dep_wait();
+  constexpr int NT = (2 * NZ + 7) / 8, nz = NZ, nout = 2 * NZ;
+  constexpr int S = HeadMmaSmem<NT>::S;
+  extern __shared__ __align__(128) unsigned char head_smem[];
+  HeadMmaSmem<NT>& sm = *reinterpret_cast<HeadMmaSmem<NT>*>(head_smem);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  for (int j = threadIdx.x; j < NT * 8; j += blockDim.x) {
+    sm.bias[j] = j < nout ? bh[j] : 0.f;
+    sm.weight[j] = j < nout ? dv.w[j < nz ? j : j - nz] : 0.f;
+  }
+  if (lane < kHmStages) tc::mbar_init(&sm.full[warp][lane], 1);
+  tc::fence_mbar_init();
+  // B fragments of the weights' three parts: [output tile][K step][register]
+  uint32_t wb[3][NT][2][2];
+#pragma unroll
+  for (int n = 0; n < NT; ++n)
+#pragma unroll
+    for (int s = 0; s < 2; ++s)
+#pragma unroll
+      for (int r = 0; r < 2; ++r) {
+        float part[3][2];
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int ci = 16 * s + 8 * r + 2 * t + e, j = 8 * n + g;
+          float w = j < nout ? wh[ci * nout + j] : 0.f;
+#pragma unroll
+          for (int q = 0; q < 3; ++q) {
+            part[q][e] = __bfloat162float(__float2bfloat16_rn(w));
+            w -= part[q][e];
+          }
+        }
+#pragma unroll
+        for (int q = 0; q < 3; ++q) wb[q][n][s][r] = bf_pack(part[q][0], part[q][1]);
+      }
+  __syncthreads();
+  float* row = sm.sums[warp];
+  const size_t plane = (size_t)H * W;
+  const int per_row = (W + 31) / 32;
+  // run (row b H + y of all images, 32 pixels) number c, c + step, ...: row and column by addition
+  const int chunks = B * H * per_row, step = gridDim.x * kHmWarps;
+  const int dq = step / per_row, dr = step - dq * per_row;
+  struct At { int by, col; };
+  auto advance = [&](At& p) {
+    p.by += dq;
+    p.col += dr;
+    if (p.col >= per_row) {
+      p.col -= per_row;
+      ++p.by;
+    }
+  };
+  float vmax = 0.f;
+  auto issue = [&](const At& p, int st) {
+    if (lane == 0) {
+      const int x0 = p.col * 32;
+      const uint32_t bytes = (uint32_t)min(32, W - x0) * 16;
+      const __nv_bfloat16* src = act + ((size_t)p.by * 4 * W + x0) * 8;
+      tc::mbar_expect_tx(&sm.full[warp][st], 4 * bytes);
+#pragma unroll
+      for (int ch = 0; ch < 4; ++ch)
+        tc::bulk_load(sm.ring[warp][st] + ch * 512, src + (size_t)ch * W * 8, bytes, &sm.full[warp][st]);
+    }
+  };
+  auto mask_of = [&](const At& p) {
+    const int x = p.col * 32 + lane;
+    return thk_mask != nullptr && x < W ? thk_mask[(size_t)p.by * W + x] : 1.f;
+  };
+  int c = blockIdx.x * kHmWarps + warp;
+  At now = {c / per_row, c - c / per_row * per_row}, next = now;
+  for (int q = 0; q < kHmStages; ++q, advance(next))
+    if (c + q * step < chunks) issue(next, q);
+  float mk = c < chunks ? mask_of(now) : 1.f;
+  int st = 0, b = 0;
+  uint32_t ph = 0;
+  // this lane's row of the four 8 x 8 matrices of an A fragment: pixel, and its plane's offset
+  const uint32_t frag = tc::smem_u32(sm.ring[warp][0]) + (uint32_t)(((lane >> 4) & 1) * 512 + ((lane & 7) + ((lane >> 3) & 1) * 8) * 16);
+  const float none[4] = {0.f, 0.f, 0.f, 0.f};
+  for (; c < chunks; c += step) {
+    const bool landed = tc::mbar_wait(&sm.full[warp][st], ph);  // bounded
+#pragma unroll
+    for (int m = 0; m < 2; ++m) {
+      uint32_t a[2][4];
+#pragma unroll
+      for (int s = 0; s < 2; ++s) ldmatrix_x4(a[s], frag + (uint32_t)(st * 2048 + s * 1024 + m * 256));
+      float d[NT][4];
+#pragma unroll
+      for (int n = 0; n < NT; ++n) mma_16816(d[n], a[0], wb[2][n][0], none);
+#pragma unroll
+      for (int q = 5; q > 0; --q)
+#pragma unroll
+        for (int n = 0; n < NT; ++n) mma_16816(d[n], a[q & 1], wb[(q - 1) / 2][n][q & 1], d[n]);
+#pragma unroll
+      for (int n = 0; n < NT; ++n)
+#pragma unroll
+        for (int r = 0; r < 4; ++r) row[(16 * m + 8 * (r >> 1) + g) * S + 8 * n + 2 * t + (r & 1)] = d[n][r];
+    }
+    __syncwarp();  // the sums are written, the stage is read
+    if (c + kHmStages * step < chunks) issue(next, st);
+    advance(next);
+    if (++st == kHmStages) {
+      st = 0;
+      ph ^= 1;
+    }
+    while (now.by >= (b + 1) * H) ++b;
+    const int x = now.col * 32 + lane;
+    const bool keep = mk > 0.f;
+    const int by = now.by;
+    advance(now);
+    if (c + step < chunks) mk = mask_of(now);
+    if (x < W) {
+      float2 v[NT * 4];
+      float nan0 = landed ? 0.f : __int_as_float(0x7fc00000);  // stays zero while all is finite
+#pragma unroll
+      for (int j = 0; j < NT * 4; ++j) {
+        v[j] = make_float2(row[lane * S + 2 * j], row[lane * S + 2 * j + 1]);
+        nan0 = fmaf(v[j].x, 0.f, fmaf(v[j].y, 0.f, nan0));
+      }
+      if (nan0 != 0.f) {
+        const uint4* px = reinterpret_cast<const uint4*>(act) + (size_t)by * 4 * W + x;
+#pragma unroll
+        for (int j = 0; j < NT * 8; ++j) {
+          float s = landed ? 0.f : __int_as_float(0x7fc00000);
+          for (int ci = 0; ci < kF && j < nout; ++ci) {
+            const uint32_t* q = reinterpret_cast<const uint32_t*>(px + (size_t)(ci >> 3) * W);
+            const uint32_t h2 = q[(ci & 7) >> 1];
+            s = fmaf((ci & 1) ? bf_hi(h2) : bf_lo(h2), wh[ci * nout + j], s);
+          }
+          ((j & 1) ? v[j >> 1].y : v[j >> 1].x) = keep ? s : 0.f;
+        }
+      }
+      // (s + bias) out_scale, or +0 where masked
+      const float2 sc = keep ? make_float2(out_scale, out_scale) : make_float2(0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < NT * 4; ++j)
+        v[j] = __ffma2_rn(__fadd2_rn(v[j], *reinterpret_cast<const float2*>(sm.bias + 2 * j)), sc, make_float2(0.f, 0.f));
+      const size_t o = (size_t)by * W + x, shift = (size_t)b * (nz - 1) * plane;
+      float* p = U + o + shift;
+#pragma unroll
+      for (int j = 0; j < NT * 8; ++j) {
+        if (j == nz) p = V + o + shift;
+        if (j < nout) *p = (j & 1) ? v[j >> 1].y : v[j >> 1].x;
+        p += plane;
+      }
+      if (dv.ubar != nullptr) {
+        float su = 0.f, sv = 0.f, u1 = 0.f, v0 = 0.f, v1 = 0.f;
+#pragma unroll
+        for (int j = 0; j < NT * 8; ++j) {
+          const float val = (j & 1) ? v[j >> 1].y : v[j >> 1].x;
+          if (j < nz) su = __fadd_rn(su, __fmul_rn(val, sm.weight[j]));
+          if (j >= nz && j < nout) sv = __fadd_rn(sv, __fmul_rn(val, sm.weight[j]));
+          if (j == nz - 1) u1 = val;
+          if (j == nz) v0 = val;
+          if (j == nout - 1) v1 = val;
+        }
+        dv.ubar[o] = su;
+        dv.vbar[o] = sv;
+        dv.ub0[o] = v[0].x;
+        dv.vb0[o] = v0;
+        dv.us0[o] = u1;
+        dv.vs0[o] = v1;
+        vmax = fmaxf(vmax, fmaxf(fabsf(su), fabsf(sv)));
+      }
+    }
+    __syncwarp();  // the sums are rewritten by the next pixels
+  }
+  if (dv.ubar != nullptr) {
+    for (int o = 16; o > 0; o >>= 1) vmax = fmaxf(vmax, __shfl_down_sync(0xffffffffu, vmax, o));
+    if (lane == 0) atomic_max_nonneg(dv.velomax, vmax);
   }
 }
 
@@ -1060,6 +1286,29 @@ extern "C" int igm_cnn_layer1_wgrad(int batch, int h, int w, int cin, const floa
   return launch_status("layer1_wgrad_kernel");
 }
 
+template <int NZ>
+static int head_fwd_mma(int batch, int h, int w, const void* act, const float* head_w, const float* head_b,
+                        float out_scale, float* U, float* V, const float* thk_mask, const HeadDerived& dv,
+                        cudaStream_t st) {
+  const long long chunks = (long long)batch * h * ((w + 31) / 32), blocks = (chunks + kHmWarps - 1) / kHmWarps;
+  IGM_CHECK_ARG(chunks < (1ll << 30) && ((uintptr_t)act & 15) == 0, IGM_ERR_BAD_SHAPE,
+                "igm_cnn_head_inference: more than 2^30 runs of 32 pixels, or an activation not 16-byte aligned");
+  const int grid = (int)(blocks < 148 * 2 ? blocks : 148 * 2);  // resident at once: a warp splits the weights once
+  constexpr size_t smem = sizeof(HeadMmaSmem<(2 * NZ + 7) / 8>);
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(head_fwd_mma_kernel<NZ>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) {
+      set_error("head_fwd_mma smem attribute: %s", cudaGetErrorString(e));
+      return IGM_ERR_CUDA;
+    }
+    configured = true;
+  }
+  launch_pdl(head_fwd_mma_kernel<NZ>, dim3(grid), dim3(kHmWarps * 32), smem, st, batch, h, w, (const __nv_bfloat16*)act,
+             head_w, head_b, out_scale, U, V, thk_mask, dv);
+  return launch_status("head_fwd_mma_kernel");
+}
+
 extern "C" int igm_cnn_head_forward(int batch, int h, int w, int nz, const void* act, const float* head_w,
                                     const float* head_b, float out_scale, float* U, float* V, const float* thk_mask,
                                     void* stream) {
@@ -1087,6 +1336,42 @@ extern "C" int igm_cnn_head_forward(int batch, int h, int w, int nz, const void*
   else
     launch_pdl(head_fwd_kernel<128>, dim3(grid), dim3(256), 0, st, batch, h, w, nz, A, head_w, head_b, out_scale, U, V, thk_mask);
   return launch_status("head_fwd_kernel");
+}
+
+extern "C" int igm_cnn_head_inference(int batch, int h, int w, int nz, const void* act, const float* head_w,
+                                            const float* head_b, float out_scale, float* U, float* V,
+                                            const float* thk_mask, const double* vert_weight, float* ubar, float* vbar,
+                                            float* uvelbase, float* vvelbase, float* uvelsurf, float* vvelsurf,
+                                            float* velomax, void* stream) {
+  IGM_CHECK_ARG(batch >= 1 && h >= 1 && w >= 1 && nz >= 1 && 2 * nz <= kF, IGM_ERR_BAD_SHAPE,
+                "igm_cnn_head_inference: bad shape (needs 2 nz <= 32)");
+  const bool derive = ubar != nullptr;
+  IGM_CHECK_ARG(act && head_w && head_b && U && V && (!derive || vert_weight), IGM_ERR_BAD_ARGUMENT,
+                "igm_cnn_head_inference: NULL argument");
+  IGM_CHECK_ARG(derive == (vbar != nullptr) && derive == (uvelbase != nullptr) && derive == (vvelbase != nullptr) &&
+                    derive == (uvelsurf != nullptr) && derive == (vvelsurf != nullptr) && derive == (velomax != nullptr),
+                IGM_ERR_BAD_ARGUMENT, "igm_cnn_head_inference: the derived outputs are all set or all NULL");
+  cudaStream_t st = as_stream(stream);
+  HeadDerived dv{};
+  for (int k = 0; k < nz && derive; ++k) dv.w[k] = (float)vert_weight[k];
+  dv.ubar = ubar; dv.vbar = vbar; dv.ub0 = uvelbase; dv.vb0 = vvelbase; dv.us0 = uvelsurf; dv.vs0 = vvelsurf;
+  dv.velomax = velomax;
+  cudaError_t e = derive ? cudaMemsetAsync(velomax, 0, sizeof(float), st) : cudaSuccess;
+  if (e != cudaSuccess) {
+    set_error("igm_cnn_head_inference: %s", cudaGetErrorString(e));
+    return IGM_ERR_CUDA;
+  }
+  switch (nz) {
+#define IGM_HEAD_MMA(Z) \
+  case Z:               \
+    return head_fwd_mma<Z>(batch, h, w, act, head_w, head_b, out_scale, U, V, thk_mask, dv, st);
+    IGM_HEAD_MMA(1) IGM_HEAD_MMA(2) IGM_HEAD_MMA(3) IGM_HEAD_MMA(4) IGM_HEAD_MMA(5) IGM_HEAD_MMA(6) IGM_HEAD_MMA(7)
+    IGM_HEAD_MMA(8) IGM_HEAD_MMA(9) IGM_HEAD_MMA(10) IGM_HEAD_MMA(11) IGM_HEAD_MMA(12) IGM_HEAD_MMA(13)
+    IGM_HEAD_MMA(14) IGM_HEAD_MMA(15) IGM_HEAD_MMA(16)
+#undef IGM_HEAD_MMA
+    default:
+      return IGM_ERR_BAD_SHAPE;
+  }
 }
 
 extern "C" size_t igm_cnn_head_partial_len(int nz) { return (size_t)kF * 2 * nz + 2 * nz + kF; }

@@ -108,9 +108,15 @@ def update_iceflow_emulated(cfg, state):
     ny, nx = f[0].shape
     buf = model.buffers(1, ny, nx, train=False)
     model.prepare_input(f, P._dx(state), [(0, 0)], ny, nx, buf)
+    capped = cfg.processes.iceflow.force_max_velbar > 0
+    if not capped and model.nout <= 32:  # the derived velocities from the head's own pass
+        U, V, d = model.forward(buf, 1, ny, nx, thk_mask=f[0], vert_weight=state.vert_weight)
+        state.U, state.V = U[0], V[0]
+        P.put_derived_velocities(state, *[t[0] for t in d[:6]], d[6])
+        return
     U, V = model.forward(buf, 1, ny, nx, thk_mask=f[0])
     state.U, state.V = U[0], V[0]
-    if cfg.processes.iceflow.force_max_velbar > 0:  # emulate.py:147-148
+    if capped:  # emulate.py:147-148
         K.force_max_velbar(state.U, state.V, cfg.processes.iceflow.force_max_velbar)
     P.set_derived_velocities(cfg, state, mask=False)
 

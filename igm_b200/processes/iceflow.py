@@ -102,8 +102,11 @@ def solve_iceflow(cfg, state, U, V):
 def set_derived_velocities(cfg, state, mask):
     """velbase / velsurf / velbar (iceflow/utils.py:21-51) and the CFL max,
     one kernel; optionally masks U, V where thk == 0 first."""
-    ub, vb, ub0, vb0, us0, vs0, vm = K.velocity_reduce(state.U, state.V, S.get(state, "thk"), state.vert_weight,
-                                                       mask=mask)
+    put_derived_velocities(state, *K.velocity_reduce(state.U, state.V, S.get(state, "thk"), state.vert_weight, mask=mask))
+
+
+def put_derived_velocities(state, ub, vb, ub0, vb0, us0, vs0, vm):
+    """Binds the fields kernels.velocity_reduce returns to the state."""
     S.put(state, "uvelbase", ub0)
     S.put(state, "vvelbase", vb0)
     S.put(state, "uvelsurf", us0)

@@ -629,6 +629,16 @@ IGM_API int igm_cnn_head_forward(int batch, int h, int w, int nz, const void* ac
                                  const float* head_b, float out_scale, float* U, float* V, const float* thk_mask,
                                  void* stream);
 
+/* The head of an inference, 2 nz <= 32: U and V as igm_cnn_head_forward (FP32
+ * sums of exact products in another order) and, from the same pass, what
+ * igm_velocity_reduce derives from them (mask 0; the same bits): ubar ..
+ * velomax all set or all NULL. */
+IGM_API int igm_cnn_head_inference(int batch, int h, int w, int nz, const void* act, const float* head_w,
+                                         const float* head_b, float out_scale, float* U, float* V,
+                                         const float* thk_mask, const double* vert_weight, float* ubar, float* vbar,
+                                         float* uvelbase, float* vvelbase, float* uvelsurf, float* vvelsurf,
+                                         float* velomax, void* stream);
+
 /* Backward of the head and of the last LeakyReLU: dpre (bf16 row-chunked) and
  * per-block partials [n_parts][igm_cnn_head_partial_len(nz)] = dWh [32][2nz],
  * dbh [2nz], db_last [32]. */

@@ -358,3 +358,37 @@ def test_conv_chain(B, H, W, nl, cin):
         if keep:
             for k in range(nl):
                 assert torch.equal(acts[k], ref[k]), k
+
+
+@pytest.mark.parametrize("B,H,W,nz", [(1, 4, 128, 10), (2, 9, 173, 16), (1, 3, 31, 1), (1, 100, 100, 5), (3, 2, 33, 4)])
+@pytest.mark.parametrize("special", [False, True])
+def test_head_with_derived_velocities(B, H, W, nz, special):
+    """The head with the derived velocities from its pass: U and V against a
+    float64 evaluation, within 1e-5 of the output's scale as the FP32 chains,
+    the rest as igm_velocity_reduce gives it from them, bit for bit; infinite and
+    NaN activations give what FP32 products give."""
+    from igm_b200 import kernels as K
+    g = torch.Generator().manual_seed(B + H + W + nz)
+    lib, st = L.lib(), L.stream_ptr()
+    a32 = bf(torch.randn(B, 32, H, W, generator=g))
+    if special:
+        a32[0, 3, 0, 0], a32[0, 5, H - 1, W - 1], a32[B - 1, 9, 1, 7] = float("inf"), float("nan"), -float("inf")
+    act = to_rc(a32).to(torch.bfloat16).cuda()
+    wh = bf(torch.randn(32, 2 * nz, generator=g)).cuda()  # two zero parts
+    bh, thk = (torch.randn(2 * nz, generator=g) * 0.1).cuda(), (torch.rand(B, H, W, generator=g) - 0.3).cuda()
+    thk[0, 0, 0] = thk[0, H - 1, W - 1] = thk[B - 1, 1, 7] = 1.0
+    w = torch.rand(nz, generator=g).double().numpy()
+    UV = [torch.full((B, nz, H, W), 7.0, device="cuda") for _ in range(2)]
+    d = [torch.full((B, H, W), 7.0, device="cuda") for _ in range(6)] + [torch.full((1,), 7.0, device="cuda")]
+    L.check(lib.igm_cnn_head_inference(B, H, W, nz, act.data_ptr(), wh.data_ptr(), bh.data_ptr(), 2.5,
+                                             UV[0].data_ptr(), UV[1].data_ptr(), thk.data_ptr(), w.ctypes.data,
+                                             *[t.data_ptr() for t in d], st))
+    same = lambda a, b: bool(((a == b) | (a.isnan() & b.isnan())).all())  # noqa: E731
+    ref = K.velocity_reduce(UV[0], UV[1], thk, w, mask=False)
+    assert all(same(x, y) for x, y in zip(d, ref))
+    y = (torch.einsum("bchw,cj->bjhw", a32.double(), wh.cpu().double()) + bh.cpu().double()[None, :, None, None]) * 2.5
+    y = torch.where((thk.cpu() > 0)[:, None], y, torch.zeros_like(y))
+    got, bad = torch.cat(UV, 1).cpu(), ~torch.isfinite(y)
+    assert bool(bad.any()) == special and torch.equal(bad, ~torch.isfinite(got))
+    assert torch.equal(got[bad].isnan(), y[bad].isnan()) and torch.equal(got[bad] > 0, y[bad] > 0)
+    assert float((got[~bad] - y[~bad]).abs().max()) <= 1e-5 * float(y[~bad].abs().max()) + 1e-6
