@@ -193,8 +193,9 @@ def ptr(t) -> int | None:
 
 def stream_ptr(stream=None) -> int:
     import torch
-    s = stream if stream is not None else torch.cuda.current_stream()
-    return s.cuda_stream
+    if stream is None:  # the current device's current stream, without building a Stream object
+        return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
+    return stream.cuda_stream
 
 
 def dtype_code(dt) -> int:
@@ -212,16 +213,18 @@ def make_grid(batch, nz, ny, nx, dx, dzeta) -> Grid:
     dz = np.asarray(dzeta, dtype=np.float64).reshape(-1)
     if nz > IGM_MAX_NZ:
         raise ValueError(f"nz={nz} > {IGM_MAX_NZ}")
-    for i, v in enumerate(dz[:IGM_MAX_NZ]):
-        g.dzeta[i] = float(v)
+    n = min(dz.size, IGM_MAX_NZ)
+    g.dzeta[:n] = dz[:n].tolist()
     return g
+
+
+_PHYSICS = dict(exp_glen=3.0, exp_weertman=3.0, regu_glen=1e-5, regu_weertman=1e-10, thr_ice_thk=0.1, min_sr=1e-20,
+                max_sr=1e20, ice_density=910.0, gravity_cst=9.81, force_negative_gravitational_energy=False)
 
 
 def make_physics(p=None, **over) -> Physics:
     """From a dict/namespace with the keys of cfg.processes.iceflow.physics."""
-    d = dict(exp_glen=3.0, exp_weertman=3.0, regu_glen=1e-5, regu_weertman=1e-10, thr_ice_thk=0.1,
-             min_sr=1e-20, max_sr=1e20, ice_density=910.0, gravity_cst=9.81,
-             force_negative_gravitational_energy=False)
+    d = dict(_PHYSICS)
     if p is not None:
         src = p if isinstance(p, dict) else vars(p)
         for k in d:

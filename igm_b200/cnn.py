@@ -119,6 +119,14 @@ class CNN:
     def _b(self, l):
         return self.params.data_ptr() + 4 * self.offsets[2 * l + 1]
 
+    def _layer_pointers(self, a, b):
+        """The forward packs and biases of the layers a .. b - 1."""
+        w0, b0 = self.wpack_f.data_ptr(), self.params.data_ptr()
+        first, each = 9 * 2 * F * 8 * 2, 9 * 4 * F * 8 * 2  # bytes of layer 0's pack and of the others'
+        wps = (C.c_void_p * (b - a))(*[w0 if l == 0 else w0 + first + (l - 1) * each for l in range(a, b)])
+        bs = (C.c_void_p * (b - a))(*[b0 + 4 * self.offsets[2 * l + 1] for l in range(a, b)])
+        return wps, bs
+
     def _w_off(self, l):
         return self.offsets[2 * l]
 
@@ -163,7 +171,7 @@ class CNN:
         B = len(windows)
         y0 = (C.c_int * B)(*[int(a) for a, _ in windows])
         x0 = (C.c_int * B)(*[int(b) for _, b in windows])
-        sc = (C.c_float * 5)(*[float(s) for s in self.scales])
+        sc = (C.c_float * 5)(*self.scales.tolist())
         rc = L.lib().igm_cnn_input(B, h, w, ny, nx, *[_p(f) for f in fields_full], float(dx), sc, y0, x0,
                                    _p(buf["X"]), *[_p(f) for f in buf["fields"]], L.stream_ptr())
         L.check(rc, "igm_cnn_input")
@@ -191,9 +199,9 @@ class CNN:
             # the 32-channel layers 1 .. L-1 in one launch (igm_conv3x3_stack)
             n = self.L - 1
             ys = [acts[l] if keep_acts else acts[l % 2] for l in range(1, self.L)]
-            outs = (C.c_void_p * n)(*[_p(y) for y in ys])
-            wps = (C.c_void_p * n)(*[self._wf(l) for l in range(1, self.L)])
-            bs = (C.c_void_p * n)(*[self._b(l) for l in range(1, self.L)])
+            pa = [_p(a) for a in acts]
+            outs = (C.c_void_p * n)(*[pa[l] if keep_acts else pa[l % 2] for l in range(1, self.L)])
+            wps, bs = self._layer_pointers(1, self.L)
             self._epoch = self._epoch % 2147483646 + 1
             hook = self.event_hook if (self.event_hook is not None and not keep_acts) else None
             if hook is not None:
@@ -233,8 +241,7 @@ class CNN:
         n = self.L // 2
         outs = [acts[2 * k + 1] if keep_acts else acts[k % 2] for k in range(n)]
         mids = (C.c_void_p * n)(*[_p(acts[2 * k]) if keep_acts else None for k in range(n)])
-        wps = (C.c_void_p * (2 * n))(*[self._wf(l) for l in range(2 * n)])
-        bs = (C.c_void_p * (2 * n))(*[self._b(l) for l in range(2 * n)])
+        wps, bs = self._layer_pointers(0, 2 * n)
         self._epoch = self._epoch % 2147483646 + 1
         hook = self.event_hook if not keep_acts else None
         if hook is not None:
@@ -264,6 +271,10 @@ class CNN:
         runs only the data-gradient chain (self.grads is then not written)."""
         lib, st = L.lib(), L.stream_ptr()
         acts = buf["acts"]
+        # device pointers of what the layers' calls below take, looked up once
+        pact, pg, perr = [_p(a) for a in acts], [_p(t) for t in buf["g"]], _p(self.err)
+        pw2, pdb2 = [_p(t) for t in buf["wpart2"]], [_p(t) for t in buf["dbpart2"]]
+        pwb = self.wpack_b.data_ptr() - 2 * 9 * 4 * F * 8  # layer l's backward pack: + l of its size
         npart, npart2 = buf["npart"], buf["npart2"]
         hw = self.params.data_ptr() + 4 * self.offsets[2 * self.L]
         hl = buf["hpart"].shape[1]
@@ -306,15 +317,13 @@ class CNN:
             if l > 0 and param_grads:
                 # both gradients of the layer in one pass (igm_conv3x3_backward), which also finishes
                 # the layer above's weight and bias gradients from the previous call's partials
-                nxt = g[1 - cur]
-                wp, dbp = buf["wpart2"][l % 2], buf["dbpart2"][l % 2]
                 if prev is None:
                     fin = (None, None, None, None)
                 else:
-                    fin = (_p(buf["wpart2"][prev % 2]), _p(buf["dbpart2"][prev % 2]), gp + 4 * self.offsets[2 * prev],
+                    fin = (pw2[prev % 2], pdb2[prev % 2], gp + 4 * self.offsets[2 * prev],
                            gp + 4 * self.offsets[2 * (prev - 1) + 1])
-                rc = lib.igm_conv3x3_backward(B, h, w, _p(gl), self._wb(l), _p(acts[l - 1]), _p(nxt), _p(dbp), _p(wp),
-                                              npart, self.alpha, _p(self.err), *fin, st)
+                rc = lib.igm_conv3x3_backward(B, h, w, pg[cur], pwb + l * 2 * 9 * 4 * F * 8, pact[l - 1], pg[1 - cur],
+                                              pdb2[l % 2], pw2[l % 2], npart, self.alpha, perr, *fin, st)
                 L.check(rc, f"igm_conv3x3_backward layer {l}")
                 prev = l
                 cur = 1 - cur
@@ -344,9 +353,8 @@ class CNN:
                     L.check(rc, "igm_cnn_wgrad_finish_split")
             if l > 0:
                 # the data gradient alone (no parameter gradients wanted)
-                nxt = g[1 - cur]
-                rc = lib.igm_conv3x3(1, B, h, w, F, _p(gl), self._wb(l), None, _p(acts[l - 1]), _p(nxt), None, npart,
-                                     self.alpha, _p(self.err), st)
+                rc = lib.igm_conv3x3(1, B, h, w, F, pg[cur], pwb + l * 2 * 9 * 4 * F * 8, None, pact[l - 1], pg[1 - cur],
+                                     None, npart, self.alpha, perr, st)
                 L.check(rc, f"igm_conv3x3 dgrad layer {l}")
                 cur = 1 - cur
 

@@ -25,7 +25,8 @@ class Workspace:
         if need == 0:
             L.check(1, f"igm_workspace_size rejected grid {grid.batch}x{grid.nz}x{grid.ny}x{grid.nx}: "
                        + L.lib().igm_last_error().decode())
-        if self.buf is None or self.buf.numel() < need or self.buf.device != torch.device(device):
+        if self.buf is None or self.buf.numel() < need or (self.buf.device != device
+                                                           and self.buf.device != torch.device(device)):
             self.buf = torch.zeros(max(need, 1 << 16), dtype=torch.uint8, device=device)
         return self.buf.data_ptr(), self.buf.numel()
 
@@ -34,7 +35,7 @@ _WS: dict = {}
 
 
 def workspace(device) -> Workspace:
-    key = str(torch.device(device))
+    key = device if isinstance(device, torch.device) else torch.device(device)
     if key not in _WS:
         _WS[key] = Workspace()
     return _WS[key]

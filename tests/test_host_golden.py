@@ -62,3 +62,23 @@ def test_time_process_matches_reference(golden):
     for t, s in zip(ts, saves):
         assert s == (abs(t - round(t)) < 1e-6), (t, s)
     assert st.continue_run == (ts[-1] < 3.0)
+
+
+def test_mass_balance_table_row_equals_numpy_interpolation():
+    """smb_simple's interpolation of a whole table row against np.interp per
+    column: the same float32 values, at, between and outside the times, for one
+    row, repeated, unsorted and non-finite tables and a long one."""
+    from igm_b200.processes.smb_simple import _interp1d, _interp_row
+    rng = np.random.default_rng(0)
+    tables = [np.sort(rng.normal(0, 100, (n, 5)).astype(np.float32), 0) for n in (1, 2, 3, 17, 64, 65)]
+    for t in tables[2:4]:
+        t[:, 1:] = rng.normal(0, 1, (t.shape[0], 4))
+    dup, uns, bad = tables[3].copy(), tables[3].copy(), tables[3].copy()
+    dup[5, 0], bad[7, 2] = dup[4, 0], np.inf
+    uns[[2, 9]] = uns[[9, 2]]
+    with np.errstate(invalid="ignore"):
+        for t in tables + [dup, uns, bad]:
+            xs = np.concatenate([t[:, 0].astype(np.float64), rng.normal(0, 150, 300), [1e9, -1e9]])
+            for x in xs.tolist():
+                ref = [_interp1d(t[:, 0], t[:, k], x) for k in range(1, 5)]
+                assert np.array_equal(np.array(_interp_row(t, x)), np.array(ref), equal_nan=True), (t.shape, x)
