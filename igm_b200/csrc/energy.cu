@@ -140,6 +140,9 @@ template <typename T> __device__ __forceinline__ T adam_step(T m_alpha, T v, T e
 }
 
 enum StencilMode { kEnergyOnly = 0, kGradient = 1, kAdamStep = 2 };
+// How a tile's boxes are loaded: by TMA (row pitch a multiple of 16 bytes), by 16-byte async copies (any
+// pitch), by one element per copy (arrays not aligned to 16 bytes).
+enum StencilLoad { kLoadElems = 0, kLoadTma = 1, kLoadRows = 2 };
 
 // Levels in flight ahead of the one being computed.  The ring also holds the
 // level being computed and the two levels whose outputs are still pending
@@ -256,7 +259,7 @@ struct TileGeo {
 // x, then y, then batch), streaming the sequence (tile, level) through one
 // ring, so the loads of a tile's first levels and its 2-D fields are issued
 // while the previous tile is still being computed.
-template <typename T, int TYP, int MODE, bool TMA, bool STD>
+template <typename T, int TYP, int MODE, int LOAD, bool STD>
 __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
     stencil_kernel(const StencilArgs<T> a, const __grid_constant__ StencilMaps maps) {
   using P = Two<T>;
@@ -273,6 +276,7 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
   constexpr int AL = Box<T>::AL;
   constexpr bool GRAD = MODE != kEnergyOnly;
   constexpr bool ADAM = MODE == kAdamStep;
+  constexpr bool TMA = LOAD == kLoadTma, ROWS = LOAD == kLoadRows;
   constexpr uint32_t kBoxBytes = NR * BW * sizeof(T);
   constexpr int kAhead = Ring<MODE>::ahead, kStages = Ring<MODE>::stages;
   static_assert(kCW == 32, "one warp per thread row");
@@ -357,9 +361,41 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
   // this thread: cells (R0, tx) and (R0 + 1, tx) of the tile; output nodes (R0 + e, tx)
   const int R0 = 2 * ty;
 
-  auto issue_fields = [&](const TileGeo& g, int fb) {  // TMA path only
-    if (tid == 0) {
-      uint64_t* bar = &SM.ffull[fb];
+  // kLoadRows: box row r of an array whose tile starts at element e0 (node (j0 - 1, i0 - 1) of the plane; rows nx
+  // apart) is copied from the 16-byte boundary at or below its first element, so its column 0 sits at box column
+  // (e0 + r nx) mod AL; a thread copies one 16-byte piece of one row of each array.  Rows of the domain only, and
+  // inside the array (`total` elements, zeros past it): what else a box holds is not used (edge tiles select zero).
+  constexpr int NPIECE = BW / AL, NPS = (NR * NPIECE + NT - 1) / NT;  // pieces of a row, and of a thread
+  const long long nodes = (long long)a.batch * (long long)plane;  // elements of a 2-D field
+  // this thread's pieces of the boxes at e0: copy(first element, box offset, bytes that exist)
+  auto pieces = [&](long long e0, int j0, long long total, auto copy) {
+#pragma unroll
+    for (int q = 0; q < NPS; ++q) {
+      const int i = tid + q * NT, pr = i / NPIECE, pc = i - pr * NPIECE;
+      if (pr >= NR) continue;
+      const long long e = e0 + (long long)pr * nx;
+      const long long at = e - (e & (AL - 1)) + pc * AL;
+      const int j = j0 - 1 + pr;
+      const bool live = j >= 0 && j < ny && at >= 0 && at < total;
+      const int n = live ? (int)(total - at < AL ? total - at : AL) : 0;
+      copy(live ? at : 0ll, pr * BW + pc * AL, n * (int)sizeof(T));
+    }
+  };
+  auto copy16 = [&](T* dst, const T* src, int bytes) {  // bytes from src, zeros up to 16
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(dst)), "l"(src), "r"(bytes) : "memory");
+  };
+
+  auto issue_fields = [&](const TileGeo& g, int fb) {  // TMA and 16-byte copies
+    uint64_t* bar = &SM.ffull[fb];
+    if (ROWS) {  // (joins the next level's group)
+      pieces((long long)g.b * (long long)plane + (long long)(g.j0 - 1) * nx + g.i0 - 1, g.j0, nodes,
+             [&](long long at, int box, int n) {
+               copy16(SM.F[fb][0] + box, a.thk + at, n);
+               copy16(SM.F[fb][1] + box, a.usurf + at, n);
+               copy16(SM.F[fb][2] + box, a.A + at, n);
+               copy16(SM.F[fb][3] + box, a.C + at, n);
+             });
+    } else if (tid == 0) {
       tc::mbar_expect_tx(bar, 4u * kBoxBytes);
       tc::tma_load_3d(SM.F[fb][0], &maps.thk, g.xs, g.j0 - 1, g.b, bar);
       tc::tma_load_3d(SM.F[fb][1], &maps.usurf, g.xs, g.j0 - 1, g.b, bar);
@@ -368,7 +404,19 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
     }
   };
   auto issue_level = [&](const TileGeo& g, int k, int st) {
-    if (TMA) {
+    if (ROWS) {
+      pieces(((long long)g.b * nz + k) * (long long)plane + (long long)(g.j0 - 1) * nx + g.i0 - 1, g.j0, nodes * nz,
+             [&](long long at, int box, int n) {
+               copy16(SM.N[st][0] + box, Ucur + at, n);
+               copy16(SM.N[st][1] + box, Vcur + at, n);
+               if (ADAM && !fresh) {
+                 copy16(SM.M[st][0] + box, a.mU + at, n);
+                 copy16(SM.M[st][1] + box, a.mV + at, n);
+                 copy16(SM.M[st][2] + box, a.vU + at, n);
+                 copy16(SM.M[st][3] + box, a.vV + at, n);
+               }
+             });
+    } else if (TMA) {
       if (tid == 0) {
         uint64_t* bar = &SM.full[st];
         const int z = g.b * nz + k;
@@ -415,7 +463,7 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
       if (++iss_i < my_tiles) ig = geo(iss_i);
     }
   };
-  if (TMA && my_tiles > 0) issue_fields(ig, 0);
+  if ((TMA || ROWS) && my_tiles > 0) issue_fields(ig, 0);
 #pragma unroll 1
   for (int q = 0; q < kAhead; ++q) issue_next();
 
@@ -431,12 +479,32 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
 #pragma unroll 1
   for (int i = 0; i < my_tiles; ++i) {
     const TileGeo g = geo(i);
-    const int fb = TMA ? (i & 1) : 0;
+    const int fb = TMA || ROWS ? (i & 1) : 0;
+    // 16-byte copies: box column of node (j0 - 1 + r, i0 - 1) is (f0 + r nx) mod AL for the fields and (f0 + r nx + k
+    // plane) mod AL for level k; nodes outside the domain are selected to zero where the tile has some
+    const int x0m = ROWS ? (int)(((long long)g.b * (long long)plane + (long long)(g.j0 - 1) * nx + g.i0 - 1) & (AL - 1)) : 0;
+    const int l0m = ROWS ? (int)((((long long)g.b * nz) * (long long)plane + (long long)(g.j0 - 1) * nx + g.i0 - 1) & (AL - 1)) : 0;
+    const int rm = nx & (AL - 1), pm = (int)(plane & (AL - 1));
+    const bool edge = ROWS && (g.j0 == 0 || g.i0 == 0 || g.j0 - 1 + NR > ny || g.i0 - 1 + NC > nx);
+    bool nod[3][2];  // this thread's nodes (rows R0 .. R0 + 2, columns tx, tx + 1) in the domain
+    if (ROWS) {
+#pragma unroll
+      for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+          nod[r][c] = g.j0 - 1 + R0 + r >= 0 && g.j0 - 1 + R0 + r < ny && g.i0 - 1 + tx + c >= 0 && g.i0 - 1 + tx + c < nx;
+    }
     if (TMA) {
       if (tid == 0 && i + 1 < my_tiles) issue_fields(geo(i + 1), fb ^ 1);
       // one thread waits for the transfer; the barrier publishes it to the CTA
       if (tid == 0 && !tc::mbar_wait(&SM.ffull[fb], (uint32_t)((i >> 1) & 1))) load_ok = false;
       __syncthreads();
+    } else if (ROWS) {
+      // this tile's fields joined the group of the level kAhead after the previous tile's first, which the
+      // levels since then have waited for unless a tile has fewer levels than that (or is the first)
+      if (i == 0 || nz <= kAhead) cp_async_wait<0>();
+      __syncthreads();
+      if (i + 1 < my_tiles) issue_fields(geo(i + 1), fb ^ 1);
     }
     // 2-D fields (element-wise path: plain loads) and B = 2 A^(-1/n) in place at in-domain nodes
 #pragma unroll
@@ -444,9 +512,9 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
       if (slot_r[q] < 0) continue;
       const int gj = g.j0 - 1 + slot_r[q], gi = g.i0 - 1 + slot_c[q];
       const bool ok = gj >= 0 && gj < ny && gi >= 0 && gi < nx;
-      const int sm = slot_r[q] * BW + slot_c[q] + g.ox;
+      const int sm = slot_r[q] * BW + slot_c[q] + (ROWS ? (x0m + slot_r[q] * rm) & (AL - 1) : g.ox);
       T Av;
-      if (TMA) {
+      if (TMA || ROWS) {
         Av = SM.F[fb][2][sm];
       } else {
         const size_t o = (size_t)g.b * plane + (ok ? (size_t)gj * nx + gi : 0);
@@ -472,15 +540,22 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
     bool cok[2], own[2], out_ok[2];
 #pragma unroll
     for (int e = 0; e < 2; ++e) {
-      const T* f0 = SM.F[fb][0] + own_sm + e * BW;
-      const T* f1 = SM.F[fb][1] + own_sm + e * BW;
-      const T* f2p = SM.F[fb][2] + own_sm + e * BW;
-      const T* f3 = SM.F[fb][3] + own_sm + e * BW;
-      const T t00 = f0[0], t01 = f0[1], t10 = f0[BW], t11 = f0[BW + 1];
-      const T u00 = f1[0], u01 = f1[1], u10 = f1[BW], u11 = f1[BW + 1];
+      T fv[4][4];  // thk, usurf, B, c at the cell's corners 00, 01, 10, 11
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+#pragma unroll
+        for (int r = 0; r < 2; ++r)
+#pragma unroll
+          for (int c = 0; c < 2; ++c) {
+            const int at = ROWS ? (R0 + e + r) * BW + tx + ((x0m + (R0 + e + r) * rm) & (AL - 1)) : own_sm + (e + r) * BW;
+            const T val = SM.F[fb][q][at + c];
+            fv[q][2 * r + c] = !ROWS || nod[e + r][c] ? val : T(0);
+          }
+      const T t00 = fv[0][0], t01 = fv[0][1], t10 = fv[0][2], t11 = fv[0][3];
+      const T u00 = fv[1][0], u01 = fv[1][1], u10 = fv[1][2], u11 = fv[1][3];
       const T th = (((t11 + t10) + t01) + t00) * quarter;
-      const T bs = (((f2p[BW + 1] + f2p[BW]) + f2p[1]) + f2p[0]) * quarter;
-      const T cv = (((f3[BW + 1] + f3[BW]) + f3[1]) + f3[0]) * quarter;
+      const T bs = (((fv[2][3] + fv[2][2]) + fv[2][1]) + fv[2][0]) * quarter;
+      const T cv = (((fv[3][3] + fv[3][2]) + fv[3][1]) + fv[3][0]) * quarter;
       const T b00 = u00 - t00, b01 = u01 - t01, b10 = u10 - t10, b11 = u11 - t11;
       // compute_gradient (staggered): 2 ds / (dx + dx), averaged over the other axis
       const T id = a.inv_dx;
@@ -528,9 +603,21 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
     P partU = zero, partV = zero;  // own-node sums of the level awaiting its finish
     int st_m1 = 0, st_m2 = 0;      // ring slots of the previous two levels
 
-    auto level_q = [&](const T* t, P& S, P& DX, P& DY) {
-      const T* p = t + own_sm;
-      const T a0 = p[0], b0 = p[1], a1 = p[BW], b1 = p[BW + 1], a2 = p[2 * BW], b2 = p[2 * BW + 1];
+    // box offset of this thread's node (R0 + r, tx) at level k
+    auto node_at = [&](int r, int k) {
+      return ROWS ? (R0 + r) * BW + tx + ((l0m + (R0 + r) * rm + k * pm) & (AL - 1)) : own_sm + r * BW;
+    };
+    auto level_q = [&](const T* t, int k, P& S, P& DX, P& DY) {
+      const T *p0 = t + node_at(0, k), *p1 = t + node_at(1, k), *p2 = t + node_at(2, k);
+      T a0 = p0[0], b0 = p0[1], a1 = p1[0], b1 = p1[1], a2 = p2[0], b2 = p2[1];
+      if (ROWS && edge) {
+        a0 = nod[0][0] ? a0 : T(0);
+        b0 = nod[0][1] ? b0 : T(0);
+        a1 = nod[1][0] ? a1 : T(0);
+        b1 = nod[1][1] ? b1 : T(0);
+        a2 = nod[2][0] ? a2 : T(0);
+        b2 = nod[2][1] ? b2 : T(0);
+      }
       const T s0 = a0 + b0, s1 = a1 + b1, s2 = a2 + b2;
       const T d0 = b0 - a0, d1 = b1 - a1, d2 = b2 - a2;
       S = {s0 + s1, s1 + s2};
@@ -566,7 +653,7 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
           a.dU[o] = gu;
           a.dV[o] = gv;
         } else if (MODE == kAdamStep) {
-          const int sm = own_sm + e * BW;
+          const int sm = node_at(e, lvl);
           const T b1c = T(1) - a.b1, b2c = T(1) - a.b2;
           T m = SM.M[st][0][sm], v = SM.M[st][2][sm];
           m += (gu - m) * b1c;
@@ -601,8 +688,8 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
       if (GRAD && !FIRST && k >= 2) finish(k - 2, st_m2);
 
       P cSu, cXu, cYu, cSv, cXv, cYv;
-      level_q(SM.N[nb][0], cSu, cXu, cYu);
-      level_q(SM.N[nb][1], cSv, cXv, cYv);
+      level_q(SM.N[nb][0], k, cSu, cXu, cYu);
+      level_q(SM.N[nb][1], k, cSv, cXv, cYv);
       if (kSkip && !FIRST && bare) {
         // Idle while every value is far from overflowing the products below (and no NaN): then they
         // are finite, and zero times them is zero.
@@ -1019,22 +1106,25 @@ static int field_maps(StencilMaps* maps, const igm_fields* f, const igm_grid* g)
   return IGM_OK;
 }
 
-// TMA needs 16-byte aligned bases and a row pitch that is a multiple of 16 bytes.
+// TMA needs 16-byte aligned bases and a row pitch that is a multiple of 16 bytes; with another pitch (three
+// widths in four) the aligned bases allow 16-byte copies, a thread's one piece per array and level where
+// the elements took 2.2 copies with an address each.  701 x 1003 x 10 FP32: energy 61.5 -> 51.3 us, energy and
+// adjoint 99 -> 70; a solver iteration at 1003 x 701 x 10 202 -> 112.  (A bulk copy per box row, issued by one
+// warp: 84, 145 and 332 us.)
 template <typename T>
-static bool tma_usable(const igm_grid* g, std::initializer_list<const void*> ptrs) {
-  if (((size_t)g->nx * sizeof(T)) % 16 != 0) return false;
+static StencilLoad stencil_load(const igm_grid* g, std::initializer_list<const void*> ptrs) {
   for (const void* p : ptrs)
-    if (p == nullptr || ((uintptr_t)p & 15) != 0) return false;
-  return true;
+    if (p == nullptr || ((uintptr_t)p & 15) != 0) return kLoadElems;
+  return ((size_t)g->nx * sizeof(T)) % 16 != 0 ? kLoadRows : kLoadTma;
 }
 
 // Persistent launch: as many CTAs as fit on the device at once (at most one per tile).
-template <typename T, int MODE, bool TMA, bool STD>
+template <typename T, int MODE, int LOAD, bool STD>
 static int launch_stencil_t(const StencilArgs<T>& s, const StencilMaps& maps, const igm_grid* g, cudaStream_t st) {
   constexpr int TYP = ThreadRows<T>::value;
   constexpr int TYC = 2 * TYP;
   constexpr size_t smem = sizeof(StencilSmem<T, TYP, MODE>) + 128;
-  auto kern = stencil_kernel<T, TYP, MODE, TMA, STD>;
+  auto kern = stencil_kernel<T, TYP, MODE, LOAD, STD>;
   static int per_sm = 0;
   if (per_sm == 0) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -1064,12 +1154,16 @@ static int launch_stencil_t(const StencilArgs<T>& s, const StencilMaps& maps, co
 }
 
 template <typename T, int MODE>
-static int launch_stencil(const StencilArgs<T>& s, const StencilMaps& maps, bool tma, const igm_grid* g,
+static int launch_stencil(const StencilArgs<T>& s, const StencilMaps& maps, StencilLoad load, const igm_grid* g,
                           cudaStream_t st) {
   const bool std_phys = s.glen3 && s.weert3 && !s.fnge;
-  if (std_phys)
-    return tma ? launch_stencil_t<T, MODE, true, true>(s, maps, g, st) : launch_stencil_t<T, MODE, false, true>(s, maps, g, st);
-  return tma ? launch_stencil_t<T, MODE, true, false>(s, maps, g, st) : launch_stencil_t<T, MODE, false, false>(s, maps, g, st);
+  if (load == kLoadTma)
+    return std_phys ? launch_stencil_t<T, MODE, kLoadTma, true>(s, maps, g, st)
+                    : launch_stencil_t<T, MODE, kLoadTma, false>(s, maps, g, st);
+  // (the row copies' variant is built for the default physics)
+  if (load == kLoadRows && std_phys) return launch_stencil_t<T, MODE, kLoadRows, true>(s, maps, g, st);
+  return std_phys ? launch_stencil_t<T, MODE, kLoadElems, true>(s, maps, g, st)
+                  : launch_stencil_t<T, MODE, kLoadElems, false>(s, maps, g, st);
 }
 
 template <typename T>
@@ -1091,15 +1185,15 @@ static int energy_t(const igm_grid* g, const igm_physics* ph, const igm_fields* 
   s.err = (int*)((char*)ws + 4);
   StencilMaps maps;
   memset(&maps, 0, sizeof(maps));
-  const bool tma = tma_usable<T>(g, {U, V, f->thk, f->usurf, f->arrhenius, f->slidingco});
-  if (tma) {
+  const StencilLoad load = stencil_load<T>(g, {U, V, f->thk, f->usurf, f->arrhenius, f->slidingco});
+  if (load == kLoadTma) {
     const int nl = g->batch * g->nz;
     if ((rc = level_map<T>(&maps.U0, U, g, nl)) || (rc = level_map<T>(&maps.V0, V, g, nl)) ||
         (rc = field_maps<T>(&maps, f, g)))
       return rc;
   }
-  if (dU) return launch_stencil<T, kGradient>(s, maps, tma, g, st);
-  return launch_stencil<T, kEnergyOnly>(s, maps, tma, g, st);
+  if (dU) return launch_stencil<T, kGradient>(s, maps, load, g, st);
+  return launch_stencil<T, kEnergyOnly>(s, maps, load, g, st);
 }
 
 template <typename T>
@@ -1136,9 +1230,9 @@ static int solver_t(const igm_grid* g, const igm_physics* ph, const igm_fields* 
   s.err = (int*)((char*)ws + 4);
   StencilMaps maps;
   memset(&maps, 0, sizeof(maps));
-  const bool tma = tma_usable<T>(g, {Uin ? Uin : U0, Vin ? Vin : V0}) &&
-      tma_usable<T>(g, {U0, V0, U1, V1, mU, mV, vU, vV, f->thk, f->usurf, f->arrhenius, f->slidingco});
-  if (tma) {
+  const StencilLoad load = stencil_load<T>(g, {Uin ? Uin : U0, Vin ? Vin : V0, U0, V0, U1, V1, mU, mV, vU, vV, f->thk,
+                                               f->usurf, f->arrhenius, f->slidingco});
+  if (load == kLoadTma) {
     const int nl = g->batch * g->nz;
     if ((rc = level_map<T>(&maps.U0, U0, g, nl)) || (rc = level_map<T>(&maps.V0, V0, g, nl)) ||
         (rc = level_map<T>(&maps.U1, U1, g, nl)) || (rc = level_map<T>(&maps.V1, V1, g, nl)) ||
@@ -1149,7 +1243,7 @@ static int solver_t(const igm_grid* g, const igm_physics* ph, const igm_fields* 
       return rc;
   }
   for (int i = 0; i < n_it; ++i) {
-    rc = launch_stencil<T, kAdamStep>(s, maps, tma, g, st);
+    rc = launch_stencil<T, kAdamStep>(s, maps, load, g, st);
     if (rc) return rc;
   }
   return IGM_OK;

@@ -235,3 +235,47 @@ def test_a_thread_without_a_context():
     t.join()
     torch.cuda.synchronize()
     assert len(got) == 1 and all(torch.equal(a, b) for a, b in zip(got[0], ref))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("shape", [(1, 3, 2, 5), (2, 2, 16, 31), (1, 4, 17, 33), (1, 5, 31, 62), (3, 3, 15, 7), (1, 2, 40, 97),
+                                   (2, 1, 33, 66), (1, 3, 47, 35)])
+def test_16_byte_copies_against_element_copies(dtype, shape):
+    """Widths whose rows do not start on 16-byte boundaries: the 16-byte copies
+    of aligned arrays against the element copies that arrays off that alignment
+    take, bit for bit: energy, gradient and three solver
+    iterations, NaN around the arrays."""
+    import ctypes as C
+    B, nz, ny, nx = shape
+    rng = np.random.default_rng(ny * nx)
+    dz = O.compute_zeta_dzeta(O.compute_levels(max(nz, 2), 4.0).double())[1].numpy()[:max(nz - 1, 1)]
+    thk = rng.uniform(0, 200, (B, ny, nx)) * (rng.random((B, ny, nx)) < 0.6)
+    data = [rng.normal(20, 10, (B, nz, ny, nx)), rng.normal(0, 10, (B, nz, ny, nx)), thk, thk + rng.uniform(2000, 2100, thk.shape),
+            rng.uniform(20, 150, thk.shape), rng.uniform(0.01, 0.1, thk.shape)]
+
+    def place(a, off):  # the array's values `off` elements past a 16-byte boundary, NaN before and after
+        buf = torch.full((a.size + 64,), float("nan"), dtype=dtype, device="cuda")
+        v = buf[16 + off:16 + off + a.size]
+        v.copy_(torch.as_tensor(a.reshape(-1)))
+        return v.view(a.shape)
+
+    got = []
+    for off in (0, 1):
+        U, V, *f = (place(a, off) for a in data)
+        terms, dU, dV = K.energy(U, V, *f, 100.0, dz, grad=True, grad_scale=1e-3)
+        terms2, _, _ = K.energy(U, V, *f, 100.0, dz)
+        g, ph, fs = K.L.make_grid(B, nz, ny, nx, 100.0, dz), K.L.make_physics(), K.fields_struct(*f)
+        W = [place(np.zeros(data[0].shape), off) for _ in range(8)]
+        ctl = torch.zeros(C.sizeof(K.L.SolverCtl), dtype=torch.uint8, device="cuda")
+        cs = torch.zeros(3, dtype=torch.float64, device="cuda")
+        ad, es = K.L.Adam(), K.L.EarlyStop()
+        ad.lr, ad.beta_1, ad.beta_2, ad.epsilon = 1.0, 0.9, 0.999, 1e-7
+        wp, wn = K.workspace(U.device).get(g, U.device)
+        K.L.check(K.L.lib().igm_solver_solve(K.L.dtype_code(dtype), C.byref(g), C.byref(ph), C.byref(fs), K.L.ptr(U), K.L.ptr(V),
+                                             *[K.L.ptr(w) for w in W], C.byref(ad), C.byref(es), 0, 3, ctl.data_ptr(),
+                                             cs.data_ptr(), wp, wn, K.L.stream_ptr()))
+        torch.cuda.synchronize()
+        assert int(K.L.SolverCtl.from_buffer_copy(ctl.cpu().numpy().tobytes()).iter) == 3
+        got.append([terms, terms2, dU, dV, cs, *[w.clone() for w in W]])
+    assert all(bool(torch.isfinite(t).all()) for t in got[0])
+    assert all(torch.equal(a, b) for a, b in zip(*got))
