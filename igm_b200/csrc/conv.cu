@@ -1291,6 +1291,12 @@ __global__ void __launch_bounds__(kConvThreads, 1) conv3x3_wgrad_kernel(const Wg
 // TMEM: 2 x 4 x 32 data-gradient columns, then 3 x 64 weight-gradient columns.
 // A stage is released when its MMAs completed (one commit) and each of the 8
 // epilogue warps has read its mask rows (one arrival each).
+//
+// A launch has a fixed part of about 9 us (one tile per CTA takes little more), and 15 of them make a
+// training step's backward.  So the weights land by a bulk copy beside the first tile's instead of through
+// registers ahead of the barrier, the layer above is finished with all of a warp's partials requested at
+// once, and the weight-gradient partials leave through shared memory as whole 128-byte rows.  Per layer at
+// 8 x 64 x 64: 22.4 us before, 19.7 now; at 1000 x 1000: 67 and 61.
 struct BwdGeom {
   static constexpr int R = 4;                           // output rows per tile
   static constexpr int C8 = 4;                          // 32 channels
@@ -1347,16 +1353,11 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_bwd_kernel(const B
   uint64_t* tfull = bars + 2 * NST;          // [NACC]
   uint64_t* tempty = bars + 2 * NST + NACC;  // [NACC]
   uint64_t* done = bars + 2 * NST + 2 * NACC;
+  uint64_t* wfull = done + 1;                // the layer's weights landed
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + G::OFF_BAR + 128);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
   grid_dep_launch();
-  grid_dep_wait();
-  {
-    const uint4* src = reinterpret_cast<const uint4*>(a.wpack);
-    uint4* dst = reinterpret_cast<uint4*>(smem + G::OFF_W);
-    for (int i = threadIdx.x; i < (int)(G::WBYTES / 16); i += kConvFwdThreads) dst[i] = src[i];
-  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < NST; ++s) {
       tc::mbar_init(&full[s], 2);                   // the two boxes' loads
@@ -1367,9 +1368,15 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_bwd_kernel(const B
       tc::mbar_init(&tempty[s], 32 * kConvEpiWarps);
     }
     tc::mbar_init(done, 1);
+    tc::mbar_init(wfull, 1);
     tc::fence_mbar_init();
   }
-  tc::fence_proxy_async_smem();
+  grid_dep_wait();
+  if (threadIdx.x == 0) {  // the weights land while the first tile does
+    tc::mbar_expect_tx(wfull, G::WBYTES);
+    tc::bulk_load(smem + G::OFF_W, a.wpack, G::WBYTES, wfull);
+  }
+  __syncwarp();
   if (warp == 0) {
     tc::tmem_alloc(tmem_slot, G::TMEM_COLS);
     tc::tmem_relinquish();
@@ -1402,8 +1409,9 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_bwd_kernel(const B
       constexpr uint32_t wg_idesc = tc::make_idesc_bf16(128, G::WN, true, true);
       const uint32_t w_lo = tc::desc_lo(sbase + G::OFF_W, kWRowsN * 16);
       const uint32_t wtm = tmem + G::DCOLS;  // weight-gradient accumulators [3][WN]
-      bool ok = true;
-      for (int it = 0, t = blockIdx.x; t < a.n_tiles; t += gridDim.x, ++it) {
+      bool ok = tc::mbar_wait(wfull, 0);
+      if (!ok) set_err(a.err, 22);
+      for (int it = 0, t = blockIdx.x; ok && t < a.n_tiles; t += gridDim.x, ++it) {
         const int s = it % NST, use = it / NST, acc = it % NACC, ause = it / NACC;
         if (!tc::mbar_wait(&tempty[acc], (ause & 1) ^ 1) || !tc::mbar_wait(&full[s], use & 1)) {
           set_err(a.err, 22);
@@ -1478,7 +1486,7 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_bwd_kernel(const B
       const int ew = warp - 2;
       for (int gi = blockIdx.x; gi < 9 * kCout; gi += gridDim.x) {
         const int ci = gi % kCout, tap = gi / kCout;
-        red[ew][lane] = finish_sum<2, 1>(a.prev_w_partial, (int)gridDim.x, ew, lane, tap % 3, tap / 3, ci, 32);
+        red[ew][lane] = finish_sum<2, 1, kFinBwdBatch>(a.prev_w_partial, (int)gridDim.x, ew, lane, tap % 3, tap / 3, ci, 32);
         asm volatile("bar.sync 1, %0;\n" ::"n"(32 * kConvEpiWarps) : "memory");
         if (ew == 0) {
           float tsum = 0.f;
@@ -1572,24 +1580,30 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_bwd_kernel(const B
       if (!ok) set_err(a.err, 25);
       tc::tc_fence_after();
     }
-    const int m = q * 32 + lane;
+    // through shared memory (the stages, once every epilogue warp has read its last mask rows), so
+    // that a store instruction writes four whole 128-byte rows and not 16 bytes of 32
+    asm volatile("bar.sync 1, %0;\n" ::"n"(32 * kConvEpiWarps) : "memory");
+    constexpr int RP = 36;  // row pitch in floats: 16-byte accesses of 8 lanes on distinct banks both ways
+    static_assert(kConvEpiWarps * 32 * RP * 4 <= NST * G::STAGE, "the exchange fits the stages");
+    float* xch = reinterpret_cast<float*>(smem) + (warp - 2) * 32 * RP;
+    const bool zero = my_tiles == 0 || !ok;
 #pragma unroll 1
     for (int dx = 0; dx < 3; ++dx) {
       const int cb = half * 32;
       uint32_t v[32];
       tc::tmem_ld32(tmem + G::DCOLS + ((uint32_t)(q * 32) << 16) + (uint32_t)(dx * G::WN + cb), v);
       tc::tmem_wait_ld();
-      float4* dst = reinterpret_cast<float4*>(a.w_partial + (((size_t)blockIdx.x * 3 + dx) * 128 + m) * G::WN + cb);
 #pragma unroll
-      for (int c = 0; c < 32; c += 4) {
-        const bool z = my_tiles == 0 || !ok;
-        float4 f4;
-        f4.x = z ? 0.f : __uint_as_float(v[c + 0]);
-        f4.y = z ? 0.f : __uint_as_float(v[c + 1]);
-        f4.z = z ? 0.f : __uint_as_float(v[c + 2]);
-        f4.w = z ? 0.f : __uint_as_float(v[c + 3]);
-        dst[c / 4] = f4;
+      for (int c = 0; c < 32; c += 4)
+        *reinterpret_cast<uint4*>(xch + lane * RP + c) = zero ? make_uint4(0, 0, 0, 0) : make_uint4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+      __syncwarp();
+      float* dst = a.w_partial + (((size_t)blockIdx.x * 3 + dx) * 128 + q * 32) * G::WN + cb;
+#pragma unroll
+      for (int r = 0; r < 32; r += 4) {
+        const int row = r + (lane >> 3), c = (lane & 7) * 4;
+        *reinterpret_cast<float4*>(dst + (size_t)row * G::WN + c) = *reinterpret_cast<const float4*>(xch + row * RP + c);
       }
+      __syncwarp();
     }
     // bias-gradient partial sums: warp reduction, then a fixed-order CTA sum below
 #pragma unroll
@@ -1761,8 +1775,8 @@ extern "C" int igm_conv3x3_backward(int batch, int height, int width, const void
                 "igm_conv3x3_backward: bad shape %dx%dx%d", batch, height, width);
   IGM_CHECK_ARG(g && wpack_bwd && x && g_prev && db_partials && w_partials && n_parts >= 1, IGM_ERR_BAD_ARGUMENT,
                 "igm_conv3x3_backward: NULL argument");
-  IGM_CHECK_ARG(((uintptr_t)g & 15) == 0 && ((uintptr_t)x & 15) == 0 && ((uintptr_t)g_prev & 15) == 0,
-                IGM_ERR_BAD_ARGUMENT, "igm_conv3x3_backward: activations must be 16-byte aligned");
+  IGM_CHECK_ARG((((uintptr_t)g | (uintptr_t)x | (uintptr_t)g_prev | (uintptr_t)wpack_bwd) & 15) == 0,
+                IGM_ERR_BAD_ARGUMENT, "igm_conv3x3_backward: activations and weights must be 16-byte aligned");
   const bool prev = prev_w_partials != nullptr;
   IGM_CHECK_ARG(prev == (prev_db_partials != nullptr) && prev == (prev_w_out != nullptr) &&
                     prev == (prev_db_out != nullptr),

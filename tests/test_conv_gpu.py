@@ -257,6 +257,13 @@ def test_conv_backward_finishes_the_previous_layer(B, H, W, npart):
     assert torch.equal(y2, y2b) and torch.equal(p2, p2b) and torch.equal(d2, d2b)
 
 
+@pytest.mark.parametrize("B,H,W,npart", [(1, 1, 1, 1), (1, 3, 40, 153), (1, 20, 130, 160)])
+def test_conv_backward_partial_counts(B, H, W, npart):
+    """The fused backward's finishing of the layer above on both sides of one
+    batch of partials (8 warps x 19), with CTAs that have no tile."""
+    test_conv_backward_finishes_the_previous_layer(B, H, W, npart)
+
+
 @pytest.mark.parametrize("B,H,W", [(1, 8, 128), (2, 9, 150), (1, 1000, 1000)])
 def test_conv1x1_wgrad_is_the_centre_tap(B, H, W):
     """igm_conv1x1_wgrad: the kw = 1 partials bit for bit as igm_conv3x3_wgrad's,
