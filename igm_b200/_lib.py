@@ -119,6 +119,7 @@ SIGNATURES = {
     "igm_conv1x1_wgrad": (I, [I, I, I, P, P, P, I, P, P]),
     "igm_conv3x3_backward": (I, [I, I, I, P, P, P, P, P, P, I, C.c_float, P, P, P, P, P, P]),
     "igm_conv3x3_stack": (I, [I, I, I, I, P, P, P, P, P, I, C.c_float, P, P]),
+    "igm_conv3x3_stack_dgrad": (I, [I, I, I, I, P, P, P, P, P, I, C.c_float, P, P]),
     "igm_conv3x3_stack_flags_len": (C.c_size_t, [I, I, I, I]),
     "igm_conv3x3_chain": (I, [I, I, I, I, I, P, P, P, P, P, P, I, C.c_float, P, P]),
     "igm_conv3x3_chain_flags_len": (C.c_size_t, [I, I, I, I]),

@@ -144,6 +144,8 @@ class CNN:
             b["X"] = act(16)  # split first-layer input (igm_cnn_input)
             if train:
                 b["g"] = [act(F), act(F)]
+                nfl = L.lib().igm_conv3x3_stack_flags_len(B, h, w, min(max(self.L - 1, 1), 16))
+                b["flags_b"] = torch.zeros(int(nfl), dtype=torch.int32, device=d)
                 b["dyb"] = act(F)  # head output gradient in bf16 (head backward on the tensor cores)
                 npart = self.n_sm
                 b["npart"] = npart          # persistent tensor-core kernels: one CTA per SM
@@ -279,6 +281,7 @@ class CNN:
         hw = self.params.data_ptr() + 4 * self.offsets[2 * self.L]
         hl = buf["hpart"].shape[1]
         g = buf["g"]
+        stacked = not param_grads and self.L > 1  # the data gradients alone: one launch for the hidden layers
         gp = self.grads.data_ptr()
         nh = F * self.nout
         if self.nout <= F:
@@ -312,7 +315,19 @@ class CNN:
                                                 gp + 4 * self.offsets[2 * (self.L - 1) + 1], 0, st), "reduce db")
         cur = 0
         prev = None  # the hidden layer whose partials the next fused call finishes
-        for l in range(self.L - 1, -1, -1):
+        if stacked:
+            for top in range(self.L - 1, 0, -16):
+                ls = range(top, max(top - 16, 0), -1)
+                n = len(ls)
+                self._epoch = self._epoch % 2147483646 + 1
+                rc = lib.igm_conv3x3_stack_dgrad(B, h, w, n, pg[cur],
+                                                 (C.c_void_p * n)(*[pg[(cur + k + 1) % 2] for k in range(n)]),
+                                                 (C.c_void_p * n)(*[pwb + l * 2 * 9 * 4 * F * 8 for l in ls]),
+                                                 (C.c_void_p * n)(*[pact[l - 1] for l in ls]), _p(buf["flags_b"]),
+                                                 self._epoch, self.alpha, perr, st)
+                L.check(rc, "igm_conv3x3_stack_dgrad")
+                cur = (cur + n) % 2
+        for l in range(0 if stacked else self.L - 1, -1, -1):
             gl = g[cur]
             if l > 0 and param_grads:
                 # both gradients of the layer in one pass (igm_conv3x3_backward), which also finishes
@@ -351,12 +366,6 @@ class CNN:
                     rc = lib.igm_cnn_wgrad_finish_split(_p(buf["wpart"]), npart, self.cin, gp + 4 * self.offsets[0],
                                                         st)
                     L.check(rc, "igm_cnn_wgrad_finish_split")
-            if l > 0:
-                # the data gradient alone (no parameter gradients wanted)
-                rc = lib.igm_conv3x3(1, B, h, w, F, pg[cur], pwb + l * 2 * 9 * 4 * F * 8, None, pact[l - 1], pg[1 - cur],
-                                     None, npart, self.alpha, perr, st)
-                L.check(rc, f"igm_conv3x3 dgrad layer {l}")
-                cur = 1 - cur
 
     def adam_step(self, lr, beta_1=0.9, beta_2=0.999, epsilon=1e-7, clipnorm=1.0):
         """Keras legacy Adam with per-variable clipnorm; repacks the weights."""

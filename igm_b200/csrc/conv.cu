@@ -390,6 +390,9 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_kernel(const ConvA
 // cooperative launch) all waits end; each is bounded all the same.  Each
 // layer's weights are copied into one of two shared-memory buffers on the
 // barrier of that layer's first tile.
+// EPI kEpiDgrad is the same stack over the data gradients, conv3x3_kernel<4, R, dgrad> per
+// layer: the epilogue multiplies with LeakyReLU' of the layer's masking activation, whose
+// rows it requests before it waits for the accumulators.
 constexpr int kStackMax = 16;
 
 struct StackArgs {
@@ -399,14 +402,15 @@ struct StackArgs {
   const __nv_bfloat16* in;        // input of layer 0 [B][H][4][W][8]
   __nv_bfloat16* out[kStackMax];  // output of layer k
   const __nv_bfloat16* wpack[kStackMax];
-  const float* bias[kStackMax];
+  const float* bias[kStackMax];          // forward
+  const __nv_bfloat16* mask[kStackMax];  // dgrad: the activation whose derivative masks layer k's output
   int* flags;                     // [nlayers][n_tiles]
   int epoch;
   float alpha;
   int* err;
 };
 
-template <int R>
+template <int R, int EPI>
 __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_stack_kernel(const StackArgs a) {
   using G = ConvGeom<4, R>;
   constexpr int NST = G::NST, NACC = G::NACC;
@@ -560,14 +564,28 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_stack_kernel(const
     bool ok = true;
     for (int k = 0; k < a.nlayers && ok; ++k) {
       float bias[kCout];
+      if (EPI == kEpiFwdLeaky) {
 #pragma unroll
-      for (int c = 0; c < kCout; ++c) bias[c] = __ldg(a.bias[k] + c);
+        for (int c = 0; c < kCout; ++c) bias[c] = __ldg(a.bias[k] + c);
+      }
       uint4* o = reinterpret_cast<uint4*>(a.out[k]);
       for (int t = first(k); t < per; t += gridDim.x, ++it) {
         const int use = it / NACC, acc = it % NACC;
         const int txi = t % a.tiles_w, rest = t / a.tiles_w;
         const int tyi = rest % a.tiles_h, b = rest / a.tiles_h;
         const int x = txi * kTW + p;
+        uint4 mk[EPI == kEpiDgrad ? RH : 1][4];
+        if (EPI == kEpiDgrad) {
+          const uint4* am = reinterpret_cast<const uint4*>(a.mask[k]);
+#pragma unroll
+          for (int rr = 0; rr < RH; ++rr) {
+            const int y = tyi * R + r0 + rr;
+            const bool in = y < a.H && x < a.W;
+            const size_t pix = in ? (((size_t)b * a.H + y) * 4) * a.W + x : 0;
+#pragma unroll
+            for (int ch = 0; ch < 4; ++ch) mk[rr][ch] = in ? am[pix + (size_t)ch * a.W] : make_uint4(0, 0, 0, 0);
+          }
+        }
         if (!tc::mbar_wait(&tfull[acc], use & 1)) {
           set_err(a.err, 34);
           ok = false;
@@ -583,10 +601,25 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_stack_kernel(const
           if (y < a.H && x < a.W) {
             const size_t pix = (((size_t)b * a.H + y) * 4) * a.W + x;
             float f[kCout];
+            if (EPI == kEpiFwdLeaky) {
 #pragma unroll
-            for (int c = 0; c < kCout; ++c) {
-              const float z = __uint_as_float(v[c]) + bias[c];
-              f[c] = z > 0.f ? z : a.alpha * z;
+              for (int c = 0; c < kCout; ++c) {
+                const float z = __uint_as_float(v[c]) + bias[c];
+                f[c] = z > 0.f ? z : a.alpha * z;
+              }
+            } else {
+#pragma unroll
+              for (int ch = 0; ch < 4; ++ch) {
+                const uint4 mv = mk[EPI == kEpiDgrad ? rr : 0][ch];
+                const uint32_t mw[4] = {mv.x, mv.y, mv.z, mv.w};
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                  const __nv_bfloat162 h2 = *reinterpret_cast<const __nv_bfloat162*>(&mw[e]);
+                  const int c = ch * 8 + e * 2;
+                  f[c] = __uint_as_float(v[c]) * (__low2float(h2) > 0.f ? 1.f : a.alpha);
+                  f[c + 1] = __uint_as_float(v[c + 1]) * (__high2float(h2) > 0.f ? 1.f : a.alpha);
+                }
+              }
             }
 #pragma unroll
             for (int ch = 0; ch < 4; ++ch) {
@@ -1595,7 +1628,8 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_bwd_kernel(const B
       tc::tmem_wait_ld();
 #pragma unroll
       for (int c = 0; c < 32; c += 4)
-        *reinterpret_cast<uint4*>(xch + lane * RP + c) = zero ? make_uint4(0, 0, 0, 0) : make_uint4(v[c], v[c + 1], v[c + 2], v[c + 3]);
+        *reinterpret_cast<uint4*>(xch + lane * RP + c) =
+            zero ? make_uint4(0, 0, 0, 0) : make_uint4(v[c], v[c + 1], v[c + 2], v[c + 3]);
       __syncwarp();
       float* dst = a.w_partial + (((size_t)blockIdx.x * 3 + dx) * 128 + q * 32) * G::WN + cb;
 #pragma unroll
@@ -1807,16 +1841,17 @@ extern "C" int igm_conv3x3_backward(int batch, int height, int width, const void
   return launch_status("conv3x3_bwd_kernel");
 }
 
-template <int R>
+template <int R, int EPI>
 static int stack_launch(int batch, int height, int width, int nlayers, const void* x, void* const* outs,
-                                 const void* const* wpacks, const float* const* biases, int* flags, int epoch,
-                                 float alpha, int* err, void* stream) {
+                        const void* const* wpacks, const float* const* biases, const void* const* masks, int* flags,
+                        int epoch, float alpha, int* err, void* stream) {
   using G = ConvGeom<4, R>;
   constexpr uint32_t SMEM = G::OFF_W + 2 * G::WBYTES + 128 + 16 + 1024;
   static_assert(SMEM <= 232448, "shared memory");
   IGM_CHECK_ARG(nlayers >= 1 && nlayers <= kStackMax, IGM_ERR_BAD_SHAPE, "igm_conv3x3_stack: 1 .. %d layers",
                 kStackMax);
-  IGM_CHECK_ARG(x && outs && wpacks && biases && flags && epoch != 0, IGM_ERR_BAD_ARGUMENT,
+  const void* const* per_layer = EPI == kEpiDgrad ? masks : reinterpret_cast<const void* const*>(biases);
+  IGM_CHECK_ARG(x && outs && wpacks && per_layer && flags && epoch != 0, IGM_ERR_BAD_ARGUMENT,
                 "igm_conv3x3_stack: NULL argument or zero epoch");
   StackArgs a{};
   a.B = batch; a.H = height; a.W = width;
@@ -1827,18 +1862,22 @@ static int stack_launch(int batch, int height, int width, int nlayers, const voi
   a.in = (const __nv_bfloat16*)x;
   IGM_CHECK_ARG(((uintptr_t)x & 15) == 0, IGM_ERR_BAD_ARGUMENT, "igm_conv3x3_stack: activations must be 16-byte aligned");
   for (int k = 0; k < nlayers; ++k) {
-    IGM_CHECK_ARG(outs[k] && wpacks[k] && biases[k] && ((uintptr_t)outs[k] & 15) == 0 && ((uintptr_t)wpacks[k] & 15) == 0,
+    IGM_CHECK_ARG(outs[k] && wpacks[k] && per_layer[k] && (((uintptr_t)outs[k] | (uintptr_t)wpacks[k]) & 15) == 0 &&
+                      (EPI == kEpiFwdLeaky || ((uintptr_t)per_layer[k] & 15) == 0),
                   IGM_ERR_BAD_ARGUMENT, "igm_conv3x3_stack: layer %d: NULL or unaligned pointer", k);
     a.out[k] = (__nv_bfloat16*)outs[k];
     a.wpack[k] = (const __nv_bfloat16*)wpacks[k];
-    a.bias[k] = biases[k];
+    if (EPI == kEpiDgrad)
+      a.mask[k] = (const __nv_bfloat16*)per_layer[k];
+    else
+      a.bias[k] = (const float*)per_layer[k];
   }
   a.flags = flags;
   a.epoch = epoch;
   a.alpha = alpha;
   a.err = err;
   static bool configured = false;
-  int rc = set_smem(conv3x3_stack_kernel<R>, SMEM, &configured);
+  int rc = set_smem(conv3x3_stack_kernel<R, EPI>, SMEM, &configured);
   if (rc) return rc;
   const int grid = a.n_tiles < sm_count() ? a.n_tiles : sm_count();
   // cooperative: every CTA resident at once, which the inter-CTA tile flags rely on
@@ -1852,7 +1891,7 @@ static int stack_launch(int batch, int height, int width, int nlayers, const voi
   attr[0].val.cooperative = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  cudaLaunchKernelEx(&cfg, conv3x3_stack_kernel<R>, a);
+  cudaLaunchKernelEx(&cfg, conv3x3_stack_kernel<R, EPI>, a);
   return launch_status("conv3x3_stack_kernel");
 }
 
@@ -1868,20 +1907,54 @@ static int stack_rows(int batch, int height, int width) {
   return kRows;
 }
 
-extern "C" int igm_conv3x3_stack(int batch, int height, int width, int nlayers, const void* x, void* const* outs,
-                                 const void* const* wpacks, const float* const* biases, int* flags, int epoch,
-                                 float alpha, int* err, void* stream) {
+template <int EPI>
+static int stack_any(int batch, int height, int width, int nlayers, const void* x, void* const* outs,
+                     const void* const* wpacks, const float* const* biases, const void* const* masks, int* flags,
+                     int epoch, float alpha, int* err, void* stream) {
   IGM_CHECK_ARG(batch >= 1 && height >= 1 && width >= 1 && batch <= 65535, IGM_ERR_BAD_SHAPE,
                 "igm_conv3x3_stack: bad shape %dx%dx%d", batch, height, width);
   switch (stack_rows(batch, height, width)) {
     case 2:
-      return stack_launch<2>(batch, height, width, nlayers, x, outs, wpacks, biases, flags, epoch, alpha, err, stream);
+      return stack_launch<2, EPI>(batch, height, width, nlayers, x, outs, wpacks, biases, masks, flags, epoch, alpha, err,
+                                  stream);
     case 4:
-      return stack_launch<4>(batch, height, width, nlayers, x, outs, wpacks, biases, flags, epoch, alpha, err, stream);
+      return stack_launch<4, EPI>(batch, height, width, nlayers, x, outs, wpacks, biases, masks, flags, epoch, alpha, err,
+                                  stream);
     default:
-      return stack_launch<kRows>(batch, height, width, nlayers, x, outs, wpacks, biases, flags, epoch, alpha, err,
-                                 stream);
+      return stack_launch<kRows, EPI>(batch, height, width, nlayers, x, outs, wpacks, biases, masks, flags, epoch, alpha,
+                                      err, stream);
   }
+}
+
+extern "C" int igm_conv3x3_stack(int batch, int height, int width, int nlayers, const void* x, void* const* outs,
+                                 const void* const* wpacks, const float* const* biases, int* flags, int epoch,
+                                 float alpha, int* err, void* stream) {
+  return stack_any<kEpiFwdLeaky>(batch, height, width, nlayers, x, outs, wpacks, biases, nullptr, flags, epoch, alpha, err,
+                                 stream);
+}
+
+extern "C" int igm_conv3x3_stack_dgrad(int batch, int height, int width, int nlayers, const void* g, void* const* outs,
+                                       const void* const* wpacks, const void* const* masks, int* flags, int epoch,
+                                       float alpha, int* err, void* stream) {
+  // One launch saves the start and the drain of each layer; a layer by itself has no barrier of its
+  // epilogue warps and no flag per tile, so these requests and stores of the masked rows run further ahead.
+  // 15 layers, a launch each against one launch: 100 x 100 139 and 94 us, 8 x 64 x 64 140 and 126, 500 x 750 273
+  // and 215, 1000 x 1000 569 and 556, 2048 x 2048 1995 and 2212: they cross at 8 tiles of 8 rows per SM.
+  IGM_CHECK_ARG(batch >= 1 && height >= 1 && width >= 1 && batch <= 65535, IGM_ERR_BAD_SHAPE,
+                "igm_conv3x3_stack_dgrad: bad shape %dx%dx%d", batch, height, width);
+  const size_t tiles = (size_t)batch * ((width + kTW - 1) / kTW) * ((height + kRows - 1) / kRows);
+  if (tiles > 8 * (size_t)sm_count()) {
+    IGM_CHECK_ARG(nlayers >= 1 && nlayers <= kStackMax && outs && wpacks && masks, IGM_ERR_BAD_ARGUMENT,
+                  "igm_conv3x3_stack_dgrad: NULL argument, or not 1 .. %d layers", kStackMax);
+    for (int k = 0; k < nlayers; ++k) {
+      const int rc = igm_conv3x3(IGM_CONV_DGRAD, batch, height, width, kCout, k ? outs[k - 1] : g, wpacks[k], nullptr,
+                                 masks[k], outs[k], nullptr, 0, alpha, err, stream);
+      if (rc) return rc;
+    }
+    return IGM_OK;
+  }
+  return stack_any<kEpiDgrad>(batch, height, width, nlayers, g, outs, wpacks, nullptr, masks, flags, epoch, alpha, err,
+                              stream);
 }
 
 extern "C" size_t igm_conv3x3_stack_flags_len(int batch, int height, int width, int nlayers) {

@@ -545,6 +545,14 @@ IGM_API int igm_conv3x3_stack(int batch, int height, int width, int nlayers, con
                               float alpha, int* err, void* stream);
 IGM_API size_t igm_conv3x3_stack_flags_len(int batch, int height, int width, int nlayers);
 
+/* The data gradients of nlayers 32-channel layers, in one launch where that is faster: from g (the
+ * gradient of a layer's pre-activation) outs[k] = igm_conv3x3's dgrad mode with wpacks[k]
+ * and act_mask masks[k] on the previous output; the same bits.  outs may alternate
+ * between two buffers, g the second of them; flags and epoch as igm_conv3x3_stack. */
+IGM_API int igm_conv3x3_stack_dgrad(int batch, int height, int width, int nlayers, const void* g, void* const* outs,
+                                    const void* const* wpacks, const void* const* masks, int* flags, int epoch,
+                                    float alpha, int* err, void* stream);
+
 /* A chain of nlayers (even) forward layers, two per pass over memory: layer 0
  * has cin_first (16 or 32) input channels, the others 32; weights and biases as
  * igm_conv3x3's forward mode.  Pass k computes layers 2k and 2k + 1: outs[k]

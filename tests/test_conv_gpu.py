@@ -399,3 +399,36 @@ def test_head_with_derived_velocities(B, H, W, nz, special):
     assert bool(bad.any()) == special and torch.equal(bad, ~torch.isfinite(got))
     assert torch.equal(got[bad].isnan(), y[bad].isnan()) and torch.equal(got[bad] > 0, y[bad] > 0)
     assert float((got[~bad] - y[~bad]).abs().max()) <= 1e-5 * float(y[~bad].abs().max()) + 1e-6
+
+
+@pytest.mark.parametrize("B,H,W,nl", [(1, 1, 1, 1), (1, 100, 100, 3), (8, 64, 64, 4), (2, 37, 300, 3), (1, 500, 750, 15),
+                                      (1, 1105, 1100, 2)])
+def test_conv_stack_dgrad(B, H, W, nl):
+    """igm_conv3x3_stack_dgrad: the data gradients of nl layers, in one launch up
+    to 8 tiles of 8 rows per SM, a launch each (no flags) above; the outputs
+    alternate between two buffers of which the second holds the input.  Bit for
+    bit what nl igm_conv3x3 dgrad calls write, twice on one flag buffer."""
+    gen = torch.Generator().manual_seed(B * 7 + H * 3 + W + nl)
+    lib, st = L.lib(), L.stream_ptr()
+    mk = lambda: to_rc(bf(torch.randn(B, 32, H, W, generator=gen))).to(torch.bfloat16).cuda()  # noqa: E731
+    g0, masks = mk(), [mk() for _ in range(nl)]
+    ws = [pack_bwd(torch.randn(3, 3, 32, 32, generator=gen) * (1.3 / np.sqrt(288))).cuda() for _ in range(nl)]
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    cur = g0
+    for k in range(nl):
+        y = torch.empty_like(g0)
+        L.check(lib.igm_conv3x3(1, B, H, W, 32, cur.data_ptr(), ws[k].data_ptr(), None, masks[k].data_ptr(), y.data_ptr(),
+                                None, 0, 0.01, err.data_ptr(), st))
+        cur = y
+    two = [torch.full_like(g0, float("nan")), torch.empty_like(g0)]
+    P = __import__("ctypes").c_void_p
+    flags = torch.zeros(int(lib.igm_conv3x3_stack_flags_len(B, H, W, nl)), dtype=torch.int32, device="cuda")
+    for epoch in (1, 2):
+        two[1].copy_(g0)
+        L.check(lib.igm_conv3x3_stack_dgrad(B, H, W, nl, two[1].data_ptr(), (P * nl)(*[two[k % 2].data_ptr() for k in range(nl)]),
+                                            (P * nl)(*[w.data_ptr() for w in ws]), (P * nl)(*[m.data_ptr() for m in masks]),
+                                            flags.data_ptr(), epoch, 0.01, err.data_ptr(), st))
+        torch.cuda.synchronize()
+        assert int(err.item()) == 0
+        assert bool((flags == (epoch if B * ((H + 7) // 8) * ((W + 127) // 128) <= 8 * 148 else 0)).all())
+        assert torch.equal(two[(nl - 1) % 2], cur)
