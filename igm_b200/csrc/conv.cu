@@ -1943,7 +1943,10 @@ extern "C" int igm_conv3x3_stack_dgrad(int batch, int height, int width, int nla
   IGM_CHECK_ARG(batch >= 1 && height >= 1 && width >= 1 && batch <= 65535, IGM_ERR_BAD_SHAPE,
                 "igm_conv3x3_stack_dgrad: bad shape %dx%dx%d", batch, height, width);
   const size_t tiles = (size_t)batch * ((width + kTW - 1) / kTW) * ((height + kRows - 1) / kRows);
-  if (tiles > 8 * (size_t)sm_count()) {
+  // A captured launch would be replayed with the same epoch, its flags already up; the layers need none.
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  cudaStreamIsCapturing(as_stream(stream), &capture);
+  if (tiles > 8 * (size_t)sm_count() || capture != cudaStreamCaptureStatusNone) {
     IGM_CHECK_ARG(nlayers >= 1 && nlayers <= kStackMax && outs && wpacks && masks, IGM_ERR_BAD_ARGUMENT,
                   "igm_conv3x3_stack_dgrad: NULL argument, or not 1 .. %d layers", kStackMax);
     for (int k = 0; k < nlayers; ++k) {

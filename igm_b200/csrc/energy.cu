@@ -1199,7 +1199,8 @@ static int energy_t(const igm_grid* g, const igm_physics* ph, const igm_fields* 
 template <typename T>
 static int solver_t(const igm_grid* g, const igm_physics* ph, const igm_fields* f, const void* Uin, const void* Vin,
                     void* U0, void* V0, void* U1, void* V1, void* mU, void* mV, void* vU, void* vV,
-                    const igm_adam* ad, const igm_early_stop* es, int n_it, int max_iter, igm_solver_ctl* ctl, double* costs, void* ws, size_t wsb,
+                    const igm_adam* ad, const igm_early_stop* es, int n_it, int max_iter, igm_solver_ctl* ctl,
+                    double* costs, void* ws, size_t wsb,
                     cudaStream_t st) {
   StencilArgs<T> s{};
   fill_common(s, g, ph, f);

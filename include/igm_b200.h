@@ -545,7 +545,8 @@ IGM_API int igm_conv3x3_stack(int batch, int height, int width, int nlayers, con
                               float alpha, int* err, void* stream);
 IGM_API size_t igm_conv3x3_stack_flags_len(int batch, int height, int width, int nlayers);
 
-/* The data gradients of nlayers 32-channel layers, in one launch where that is faster: from g (the
+/* The data gradients of nlayers 32-channel layers, in one launch where that is faster (and
+ * the stream is not being captured): from g (the
  * gradient of a layer's pre-activation) outs[k] = igm_conv3x3's dgrad mode with wpacks[k]
  * and act_mask masks[k] on the previous output; the same bits.  outs may alternate
  * between two buffers, g the second of them; flags and epoch as igm_conv3x3_stack. */

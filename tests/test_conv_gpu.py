@@ -432,3 +432,36 @@ def test_conv_stack_dgrad(B, H, W, nl):
         assert int(err.item()) == 0
         assert bool((flags == (epoch if B * ((H + 7) // 8) * ((W + 127) // 128) <= 8 * 148 else 0)).all())
         assert torch.equal(two[(nl - 1) % 2], cur)
+
+
+def test_conv_stack_dgrad_captured():
+    """Under stream capture igm_conv3x3_stack_dgrad takes a launch per layer: a
+    graph replayed twice gives the bits of igm_conv3x3's dgrad calls."""
+    gen = torch.Generator().manual_seed(3)
+    lib, nl, P = L.lib(), 3, __import__("ctypes").c_void_p
+    mk = lambda: to_rc(bf(torch.randn(1, 32, 40, 150, generator=gen))).to(torch.bfloat16).cuda()  # noqa: E731
+    g0, masks, two = mk(), [mk() for _ in range(nl)], [mk(), mk()]
+    w = pack_bwd(torch.randn(3, 3, 32, 32, generator=gen) * (1.3 / np.sqrt(288))).cuda()
+    err = torch.zeros(1, dtype=torch.int32, device="cuda")
+    flags = torch.zeros(int(lib.igm_conv3x3_stack_flags_len(1, 40, 150, nl)), dtype=torch.int32, device="cuda")
+
+    def call():
+        L.check(lib.igm_conv3x3_stack_dgrad(1, 40, 150, nl, g0.data_ptr(), (P * nl)(*[two[k % 2].data_ptr() for k in range(nl)]),
+                                            (P * nl)(*([w.data_ptr()] * nl)), (P * nl)(*[m.data_ptr() for m in masks]),
+                                            flags.data_ptr(), 1, 0.01, err.data_ptr(), L.stream_ptr()))
+
+    ref = g0
+    for m in masks:
+        y = torch.empty_like(g0)
+        L.check(lib.igm_conv3x3(1, 1, 40, 150, 32, ref.data_ptr(), w.data_ptr(), None, m.data_ptr(), y.data_ptr(), None, 0,
+                                0.01, err.data_ptr(), L.stream_ptr()))
+        ref = y
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call()
+    for _ in range(2):
+        two[0].fill_(float("nan"))
+        graph.replay()
+        torch.cuda.synchronize()
+        assert int(err.item()) == 0 and torch.equal(two[0], ref)
