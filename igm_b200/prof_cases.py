@@ -5,8 +5,8 @@ Stencil (energy, energy + adjoint, one fused Adam iteration), transport and
 the vertical velocity at 1500 x 1500 x Nz 10 in FP32; the data-assimilation
 cost/gradient, flow direction and upwind divergence at 1500 x 1500 in FP32;
 the tensor-core convolution (forward, dgrad, wgrad, the fused backward) at
-batch 2 x 1000 x 1000 x 32 channels, and the forward stack of 15 such layers
-at batch 1.
+batch 2 x 1000 x 1000 x 32 channels, and at batch 1 the forward and the
+data-gradient stack of 15 such layers, the 16-layer chain and the inference head.
 
 ``python -m igm_b200.prof_cases assimilation_iteration`` instead sets up the
 data-assimilation loop on the 1000 x 1000 x Nz 10 glacier tongue (default
@@ -102,6 +102,21 @@ def main():
     flags = torch.zeros(int(lib.igm_conv3x3_stack_flags_len(1, H, W, nl)), dtype=torch.int32, device="cuda")
     L.check(lib.igm_conv3x3_stack(1, H, W, nl, x.data_ptr(), outs, wps, bss, flags.data_ptr(), 1, 0.01,
                                   err.data_ptr(), s), "conv stack")
+    # the data gradients of the same layers in the stack's kernel; the inference's chain (16 layers from the
+    # 16-channel input, two per pass) and its head
+    msk = (C.c_void_p * nl)(*([x.data_ptr()] * nl))
+    L.check(lib.igm_conv3x3_stack_dgrad(1, H, W, nl, y2.data_ptr(), outs, wps, msk, flags.data_ptr(), 2, 0.01,
+                                        err.data_ptr(), s), "conv dgrad stack")
+    nl, x16 = 16, torch.randn(1, H, 2, W, 8, device="cuda").to(torch.bfloat16)
+    cflags = torch.zeros(int(lib.igm_conv3x3_chain_flags_len(1, H, W, nl)), dtype=torch.int32, device="cuda")
+    L.check(lib.igm_conv3x3_chain(1, H, W, nl, 16, x16.data_ptr(), (C.c_void_p * (nl // 2))(),
+                                  (C.c_void_p * (nl // 2))(*[(y, y2)[k % 2].data_ptr() for k in range(nl // 2)]),
+                                  (C.c_void_p * nl)(*([wp.data_ptr()] * nl)), (C.c_void_p * nl)(*([bias.data_ptr()] * nl)),
+                                  cflags.data_ptr(), 1, 0.01, err.data_ptr(), s), "conv chain")
+    hw, hb = torch.randn(32, 2 * nz, device="cuda"), torch.zeros(2 * nz, device="cuda")
+    hU, hV = (torch.empty(nz, H, W, device="cuda") for _ in range(2))
+    L.check(lib.igm_cnn_head_inference(1, H, W, nz, y.data_ptr(), hw.data_ptr(), hb.data_ptr(), 1.0, hU.data_ptr(),
+                                       hV.data_ptr(), None, None, *[None] * 7, s), "head inference")
     torch.cuda.synchronize()
     if int(err.item()) != 0:
         raise RuntimeError(f"kernel error flag {int(err.item())}")
