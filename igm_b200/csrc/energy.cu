@@ -266,10 +266,7 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
   using SmemT = StencilSmem<T, TYP, MODE>;
   // STD: the default physics (Glen n = 3, Weertman m = 3, gravitational energy not forced
   // negative), fixed at compile time so that its branches and generic powers drop out
-  // Bare warps skip their layers, but not in the fused iteration: it is bound by its loads, gains nothing
-  // where half of the ice is missing (147 us at 1000 x 1000 x 10 with and without) and loses where all
-  // ground is covered (163 us with, 153 without).
-  constexpr bool kSkip = STD && MODE != kAdamStep;
+  constexpr bool kSkip = STD;  // bare warps skip their layers
   const bool glen3 = STD || a.glen3, weert3 = STD || a.weert3, fnge = !STD && a.fnge;
   constexpr int TYC = 2 * TYP;  // cell rows per tile
   constexpr int NT = kCW * TYP;
