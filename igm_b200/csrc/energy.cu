@@ -37,6 +37,7 @@
 // to finish sums them in a fixed order (deterministic for a given device) and,
 // in solver mode, runs EarlyStopping on the device.
 #include <stdarg.h>
+#include <cmath>
 
 #include <string.h>
 
@@ -166,6 +167,8 @@ struct StencilArgs {
   T dx, inv_dx;
   T dzeta[IGM_MAX_NZ];
   T inv_dzeta[IGM_MAX_NZ];
+  T inv_dzeta_max;  // the largest |inv_dzeta| of the layers
+  int bare_skip;    // bare ground may be skipped: several levels, and constants whose products stay finite
   // physics
   T q, inv_p, regu2, sr_lo, sr_hi, thr, Kg, inv_n, s_w, inv_sw, regw2;
   // working units of the kernel: sr2 = k2 sr2w (k2 = 1/(32 dx^2)), clip bounds of sr2w,
@@ -266,7 +269,9 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
   using SmemT = StencilSmem<T, TYP, MODE>;
   // STD: the default physics (Glen n = 3, Weertman m = 3, gravitational energy not forced
   // negative), fixed at compile time so that its branches and generic powers drop out
-  // bare warps skip their layers; not the FP32 fused iteration, load-bound: all ice 163 us with, 153 without
+  // Bare warps skip their layers, but not in the FP32 iteration, where the zero steps (adam_step) already save what
+  // bare ground can: with the skip half ice at 1000 x 1000 x 10 is 147 us either way and all ice 163 us, without it
+  // 153.  FP64 there: half ice 290 us with it and 324 without, all ice 351 and 348.
   constexpr bool kSkip = STD && (MODE != kAdamStep || sizeof(T) == 8);
   const bool glen3 = STD || a.glen3, weert3 = STD || a.weert3, fnge = !STD && a.fnge;
   constexpr int TYC = 2 * TYP;  // cell rows per tile
@@ -591,11 +596,23 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
     const long long obase = ((long long)g.b * nz) * (long long)plane +
                             (long long)(g.j0 - 1 + R0) * nx + (g.i0 - 1 + tx);
 
-    // No ice in this warp's cells (warp-uniform): their shear and gravity energies and gradients are
-    // exactly zero, whatever finite velocities a level holds, so its layers are skipped.
-    // Half of a valley, and more of most domains, is such ground.  Half of it ice: energy and adjoint at
-    // 1000 x 1000 x 10 98 -> 90 us, energy 51 -> 47; FP64 at 400 x 400 43.2 -> 34.6 and 26.8 -> 22.7.
-    const bool bare = kSkip && nz > 1 && __all_sync(0xffffffffu, thks.x == T(0) && thks.y == T(0));
+    // No ice in this warp's cells (warp-uniform): the factors that their shear and gravity energies and
+    // gradients carry are zero, and so are these wherever what is multiplied with them is finite.  A rate
+    // factor, a surface slope or a gradient scale that is not finite makes a factor 0 x inf or NaN, not zero;
+    // `reach` bounds the velocity derivatives per unit of velocity.  Then two levels of modest velocities (below)
+    // leave nothing to add for the layer between them, and it is skipped.
+    // Half of a valley, and more of most domains, is such ground.  Half of it ice, without the skip and with it:
+    // energy and adjoint at 1000 x 1000 x 10 98.3 and 90.8 us, energy 51.7 and 50.2; FP64 at 400 x 400 43.6 and 39.1,
+    // 27.0 and 23.9.
+    bool bare = kSkip && a.bare_skip != 0 && __all_sync(0xffffffffu, thks.x == T(0) && thks.y == T(0));
+    if (kSkip && bare) {
+      const P fs = GRAD ? gshc : esc, fx = GRAD ? gxc : egc * ssx, fy = GRAD ? gyc : egc * ssy;
+      const P reach = rzc * two(a.inv_dzeta_max) * P{T(1) + fabs(sbx.x) + fabs(sby.x), T(1) + fabs(sbx.y) + fabs(sby.y)} +
+                      P{fabs(ssx.x) + fabs(ssy.x), fabs(ssx.y) + fabs(ssy.y)};
+      bare = __all_sync(0xffffffffu, fs.x == T(0) && fs.y == T(0) && fx.x == T(0) && fx.y == T(0) && fy.x == T(0) &&
+                                         fy.y == T(0) && reach.x < T(1e8) && reach.y < T(1e8));
+    }
+    bool calm = false;  // the previous level's velocities were modest in the whole warp
     bool pending = true;  // the adjoint awaiting its flush may be non-zero (warp-uniform)
     P e_sh = zero, eGu = zero, eGv = zero, e_slid = zero, e_gf = zero;
     // previous level's corner sums, pending adjoint of the previous level
@@ -691,12 +708,13 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
       P cSu, cXu, cYu, cSv, cXv, cYv;
       level_q(SM.N[nb][0], k, cSu, cXu, cYu);
       level_q(SM.N[nb][1], k, cSv, cXv, cYv);
-      if (kSkip && !FIRST && bare) {
-        // Idle while every value is far from overflowing the products below (and no NaN): then they
-        // are finite, and zero times them is zero.
+      if (kSkip && bare) {
+        // Modest (and no NaN): X .. W, uz, vz below 4e18, the sum of their squares finite in FP32.
         const P big = {fabs(cSu.x) + fabs(cXu.x) + fabs(cYu.x) + fabs(cSv.x) + fabs(cXv.x) + fabs(cYv.x),
                        fabs(cSu.y) + fabs(cXu.y) + fabs(cYu.y) + fabs(cSv.y) + fabs(cXv.y) + fabs(cYv.y)};
-        if (__all_sync(0xffffffffu, big.x < T(1e10) && big.y < T(1e10))) {
+        const bool both = calm;
+        calm = __all_sync(0xffffffffu, big.x < T(1e10) && big.y < T(1e10));
+        if (!FIRST && both && calm) {
           if (GRAD) {
             if (pending) {
               flush(k - 1, gSu, gXu, gYu, 0, partU);
@@ -987,6 +1005,14 @@ static void fill_common(StencilArgs<T>& s, const igm_grid* g, const igm_physics*
   for (int l = 0; l < IGM_MAX_NZ; ++l) {
     s.dzeta[l] = (T)g->dzeta[l];
     s.inv_dzeta[l] = g->dzeta[l] != 0.0 ? (T)(1.0 / g->dzeta[l]) : T(0);
+  }
+  // the regularisation bounds the viscosity factor (to 1e6, its fourth power to 1e24) and finite layers
+  // the weights; with less, products of the skipped layers could overflow
+  s.bare_skip = g->nz > 1 && ph->regu_glen * ph->regu_glen >= 1e-18;
+  for (int l = 0; l < g->nz - 1; ++l) {
+    const T inv = std::fabs(s.inv_dzeta[l]);
+    if (!(std::fabs(g->dzeta[l]) < 1e6) || !std::isfinite(inv)) s.bare_skip = 0;
+    if (inv > s.inv_dzeta_max) s.inv_dzeta_max = inv;
   }
   const double n = ph->exp_glen, m = ph->exp_weertman;
   const double p = 1.0 + 1.0 / n;

@@ -279,3 +279,38 @@ def test_16_byte_copies_against_element_copies(dtype, shape):
         got.append([terms, terms2, dU, dV, cs, *[w.clone() for w in W]])
     assert all(bool(torch.isfinite(t).all()) for t in got[0])
     assert all(torch.equal(a, b) for a, b in zip(*got))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("nx", [64, 66])
+@pytest.mark.parametrize("what,value,level", [("U", float("nan"), 0), ("V", float("inf"), 0), ("U", 1e25, 0), ("U", float("nan"), 2),
+                                              ("V", float("inf"), 4), ("arrhenius", float("nan"), 0), ("arrhenius", 0.0, 0),
+                                              ("usurf", float("nan"), 0), ("usurf", float("inf"), 0),
+                                              ("scale", float("nan"), 0), ("scale", float("inf"), 0), ("dzeta", float("nan"), 2)])
+def test_bare_ground_hides_nothing(dtype, nx, what, value, level):
+    """A value that is not finite far off the ice (row 60; ice in rows 16 ..
+    47) shows in the same energy terms and at the same nodes of the gradient as
+    with a trace of ice (1e-30 m) on the bare ground, where no layer is skipped."""
+    ny, nz = 70, 5
+    st = O.valley_glacier(ny, nx, 100.0, seed=5, varying_coeffs=True)
+    rng = np.random.default_rng(6)
+    ice = np.zeros((ny, nx))
+    ice[16:48] = rng.uniform(50, 150, (32, nx))
+    f = {"U": rng.normal(20, 10, (nz, ny, nx)), "V": rng.normal(0, 10, (nz, ny, nx)), "usurf": st["topg"] + ice,
+         "arrhenius": np.array(st["arrhenius"], np.float64), "slidingco": st["slidingco"]}
+    dz = O.compute_zeta_dzeta(O.compute_levels(nz, 4.0).double())[1].numpy()
+    scale = 1e-3
+    if what == "scale":
+        scale = value
+    elif what == "dzeta":
+        dz[level] = value
+    else:
+        f[what][(level, 60, 33) if what in "UV" else (60, 33)] = value
+    got = []
+    for thk in (ice, np.where(ice > 0, ice, 1e-30)):
+        args = [dev(a, dtype) for a in (f["U"], f["V"], thk, f["usurf"], f["arrhenius"], f["slidingco"])]
+        terms, dU, dV = K.energy(*args, 100.0, dz, grad=True, grad_scale=scale)
+        only, _, _ = K.energy(*args, 100.0, dz)
+        got.append([torch.isfinite(t).cpu() for t in (terms, only, dU, dV)])
+    for i, (a, b) in enumerate(zip(*got)):
+        assert torch.equal(a, b), (i, (a != b).nonzero()[:8].tolist())
