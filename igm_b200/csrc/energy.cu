@@ -602,8 +602,8 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
     // `reach` bounds the velocity derivatives per unit of velocity.  Then two levels of modest velocities (below)
     // leave nothing to add for the layer between them, and it is skipped.
     // Half of a valley, and more of most domains, is such ground.  Half of it ice, without the skip and with it:
-    // energy and adjoint at 1000 x 1000 x 10 98.3 and 90.8 us, energy 51.7 and 50.2; FP64 at 400 x 400 43.6 and 39.1,
-    // 27.0 and 23.9.
+    // energy and adjoint at 1000 x 1000 x 10 98.3 and 87.9 us, energy 51.7 and 49.6; FP64 at 400 x 400 43.6 and 38.7,
+    // 27.0 and 23.2.
     bool bare = kSkip && a.bare_skip != 0 && __all_sync(0xffffffffu, thks.x == T(0) && thks.y == T(0));
     if (kSkip && bare) {
       const P fs = GRAD ? gshc : esc, fx = GRAD ? gxc : egc * ssx, fy = GRAD ? gyc : egc * ssy;
@@ -692,8 +692,9 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
 
     // one level of the stream; the first level (sliding, no layer below it) is peeled
     // off at compile time so that the steady-state loop carries no branches on k
-    auto level = [&](const int k, auto first_tag) {
+    auto level = [&](const int k, auto first_tag, auto test_tag) {
       constexpr bool FIRST = decltype(first_tag)::value;
+      constexpr int TEST = decltype(test_tag)::value;  // may the warp skip layers: 0 no, 1 yes, 2 where it is bare
       const int nb = cons_st;
       if (TMA) {
         // level k landed: one thread waits (the others spend no issue slots polling)
@@ -701,14 +702,17 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
       } else {
         cp_async_wait<kAhead - 1>();  // this thread's copies of level k have landed
       }
-      __syncthreads();  // level k visible to all; every thread is done with the previous iteration
+      // level k visible to all; every thread is done with the previous iteration.  (Written out: a CTA's warps
+      // may wait here in different loops, which the instruction allows, being counted by warps, and __syncthreads
+      // does not.)
+      asm volatile("barrier.sync.aligned 0;\n" ::: "memory");
       issue_next();
       if (GRAD && !FIRST && k >= 2) finish(k - 2, st_m2);
 
       P cSu, cXu, cYu, cSv, cXv, cYv;
       level_q(SM.N[nb][0], k, cSu, cXu, cYu);
       level_q(SM.N[nb][1], k, cSv, cXv, cYv);
-      if (kSkip && bare) {
+      if (TEST == 1 || (TEST == 2 && bare)) {
         // Modest (and no NaN): X .. W, uz, vz below 4e18, the sum of their squares finite in FP32.
         const P big = {fabs(cSu.x) + fabs(cXu.x) + fabs(cYu.x) + fabs(cSv.x) + fabs(cXv.x) + fabs(cYv.x),
                        fabs(cSu.y) + fabs(cXu.y) + fabs(cYu.y) + fabs(cSv.y) + fabs(cXv.y) + fabs(cYv.y)};
@@ -859,9 +863,22 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
         cons_ph ^= 1u;
       }
     };
-    level(0, std::true_type{});
+    // Energy and adjoint: warps with ice run a loop of their own, without the test (the barriers count warps,
+    // whichever loop they are in).  With one loop for both, ice everywhere, 1000 x 1000 x 10: the adjoint 103 us,
+    // now 98.2, the energy 55.8 and 53.7.  The FP64 iteration keeps one (two: half ice 291 us, all ice 355; one:
+    // 290 and 351).
+    using InLoop = std::integral_constant<int, kSkip && ADAM ? 2 : 0>;
+    using Bare = std::integral_constant<int, kSkip && !ADAM ? 1 : 0>;
+    constexpr int kBareUnroll = GRAD ? 1 : 2;  // unrolled by two, the adjoint with ice everywhere takes 99.0 us
+    if (Bare::value && bare) {
+      level(0, std::true_type{}, Bare{});
+#pragma unroll kBareUnroll
+      for (int k = 1; k < nz; ++k) level(k, std::false_type{}, Bare{});
+    } else {
+      level(0, std::true_type{}, InLoop{});
 #pragma unroll 2
-    for (int k = 1; k < nz; ++k) level(k, std::false_type{});
+      for (int k = 1; k < nz; ++k) level(k, std::false_type{}, InLoop{});
+    }
     if (GRAD) {
       __syncthreads();
       if (nz >= 2) finish(nz - 2, st_m2);
