@@ -136,8 +136,11 @@ template <> __device__ __forceinline__ Two<float> rcbrt2<float>(Two<float> x) {
 // ice every node's gradient and moments are zero, which the square root and the
 // division would each take their slow paths for: an iteration at 1000 x 1000 x
 // 10, half of it ice, 173.5 -> 146 us, at 100 x 100 25.9 -> 22.1.
-template <typename T> __device__ __forceinline__ T adam_step(T m_alpha, T v, T eps) {
-  return m_alpha == T(0) ? T(0) : m_alpha / (Math<T>::sqrt(v) + eps);
+// With epsilon 0 that step is 0 / 0, not zero: such a solve takes the element
+// copies' variant, the only one that looks at epsilon (ANY_EPS; in the others
+// the look took 1 % of an iteration).
+template <typename T, bool ANY_EPS> __device__ __forceinline__ T adam_step(T m_alpha, T v, T eps) {
+  return m_alpha == T(0) && (!ANY_EPS || eps > T(0)) ? T(0) : m_alpha / (Math<T>::sqrt(v) + eps);
 }
 
 enum StencilMode { kEnergyOnly = 0, kGradient = 1, kAdamStep = 2 };
@@ -677,14 +680,14 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
           v += (gu * gu - v) * b2c;
           a.mU[o] = m;
           a.vU[o] = v;
-          Unxt[o] = SM.N[st][0][sm] - adam_step<T>(m * alpha, v, a.eps);
+          Unxt[o] = SM.N[st][0][sm] - adam_step<T, LOAD == kLoadElems>(m * alpha, v, a.eps);
           m = SM.M[st][1][sm];
           v = SM.M[st][3][sm];
           m += (gv - m) * b1c;
           v += (gv * gv - v) * b2c;
           a.mV[o] = m;
           a.vV[o] = v;
-          Vnxt[o] = SM.N[st][1][sm] - adam_step<T>(m * alpha, v, a.eps);
+          Vnxt[o] = SM.N[st][1][sm] - adam_step<T, LOAD == kLoadElems>(m * alpha, v, a.eps);
         }
       }
     };
@@ -1275,8 +1278,9 @@ static int solver_t(const igm_grid* g, const igm_physics* ph, const igm_fields* 
   s.err = (int*)((char*)ws + 4);
   StencilMaps maps;
   memset(&maps, 0, sizeof(maps));
-  const StencilLoad load = stencil_load<T>(g, {Uin ? Uin : U0, Vin ? Vin : V0, U0, V0, U1, V1, mU, mV, vU, vV, f->thk,
-                                               f->usurf, f->arrhenius, f->slidingco});
+  StencilLoad load = stencil_load<T>(g, {Uin ? Uin : U0, Vin ? Vin : V0, U0, V0, U1, V1, mU, mV, vU, vV, f->thk,
+                                         f->usurf, f->arrhenius, f->slidingco});
+  if (!(s.eps > T(0))) load = kLoadElems;  // adam_step
   if (load == kLoadTma) {
     const int nl = g->batch * g->nz;
     if ((rc = level_map<T>(&maps.U0, U0, g, nl)) || (rc = level_map<T>(&maps.V0, V0, g, nl)) ||

@@ -178,3 +178,16 @@ def test_start_is_read_in_place(n, offset):
     for got, ref in zip((Ur, Vr), W[2 * (n % 2):2 * (n % 2) + 2]):
         assert torch.equal(got, torch.where(ice, ref, torch.zeros_like(ref)))
     np.testing.assert_array_equal(costs, cs.cpu().numpy()[:n])
+
+
+def test_zero_epsilon_without_a_gradient_is_not_a_number():
+    """Adam's step 0 / (sqrt(0) + 0) of a node whose gradient is zero: with
+    epsilon 0 the solve stops, as the division gives it."""
+    st = O.valley_glacier(40, 36, 100.0, seed=4)
+    dz = O.compute_zeta_dzeta(O.compute_levels(5, 4.0))[1].numpy()
+    Z = torch.zeros((5, 40, 36), device="cuda")
+    f = [dev(st[k]) for k in ["thk", "usurf", "arrhenius", "slidingco"]]
+    assert not bool((f[0] > 0).all())
+    with pytest.raises(L.IgmError) as ei:
+        DeviceAdamSolver(epsilon=0.0).solve(Z, Z, *f, 100.0, dz, nbitmax=5)
+    assert ei.value.status == 3
