@@ -32,9 +32,10 @@ class IceflowEnergy(torch.autograd.Function):
     def backward(ctx, gout):
         U, V, thk, usurf, arrhenius, slidingco = ctx.saved_tensors
         dx, dzeta, phys, count = ctx.args
-        # the incoming gradient is read by the kernel: no wait for the forward here
-        _, dU, dV = K.energy(U, V, thk, usurf, arrhenius, slidingco, dx, dzeta, phys, grad=True, grad_out=gout.contiguous(),
-                             grad_count=count)
+        # the incoming gradient is read by the kernel, from memory (a lazily negated view holds -gout there): no wait
+        # for the forward here
+        _, dU, dV = K.energy(U, V, thk, usurf, arrhenius, slidingco, dx, dzeta, phys, grad=True,
+                             grad_out=gout.resolve_neg().contiguous(), grad_count=count)
         return dU, dV, None, None, None, None, None, None, None
 
 

@@ -314,3 +314,20 @@ def test_bare_ground_hides_nothing(dtype, nx, what, value, level):
         got.append([torch.isfinite(t).cpu() for t in (terms, only, dU, dV)])
     for i, (a, b) in enumerate(zip(*got)):
         assert torch.equal(a, b), (i, (a != b).nonzero()[:8].tolist())
+
+
+def test_backward_of_a_lazily_negated_gradient():
+    """The incoming gradient of an imaginary part of a conjugate is a view whose
+    memory holds the opposite sign."""
+    from igm_b200.energy import iceflow_energy
+    ny, nx, nz = 17, 20, 3
+    st = O.valley_glacier(ny, nx, 100.0, seed=7, varying_coeffs=True)
+    rng = np.random.default_rng(8)
+    f = [dev(st[k], torch.float32) for k in ["thk", "usurf", "arrhenius", "slidingco"]]
+    dz = O.compute_zeta_dzeta(O.compute_levels(nz, 4.0))[1].numpy()
+    U, V = (dev(rng.normal(5, 9, (nz, ny, nx)), torch.float32).requires_grad_(True) for _ in range(2))
+    g = torch.complex(torch.zeros((), device="cuda"), torch.full((), 0.5, device="cuda")).conj().imag
+    assert g.is_neg() and float(g) == -0.5
+    got = torch.autograd.grad(iceflow_energy(U, V, *f, 100.0, dz), [U, V], grad_outputs=g)
+    ref = torch.autograd.grad(iceflow_energy(U, V, *f, 100.0, dz), [U, V], grad_outputs=g.resolve_neg())
+    assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
