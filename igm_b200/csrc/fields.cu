@@ -744,11 +744,14 @@ static int vert_flow_t(int nz, int ny, int nx, double dx, const void* U, const v
   a.nz = nz; a.ny = ny; a.nx = nx;
   a.dx = (T)dx;
   a.rdx = T(1) / a.dx;
+  bool weightless = true;  // up to level k
   for (int k = 0; k < nz; ++k) {
     a.ddz[k] = k > 0 ? (T)levels[k] - (T)levels[k - 1] : T(0);
     a.w[k] = (T)vert_weight[k];
     a.sw[k] = k > 0 ? a.sw[k - 1] + a.w[k] : a.w[k];
-    a.rsw[k] = T(1) / a.sw[k];  // host IEEE division in T
+    weightless = weightless && a.w[k] == T(0);
+    // host IEEE division in T; below the first weight sum and mean are zero (div_dx of 0 by 1 / 0 would be NaN)
+    a.rsw[k] = weightless ? T(0) : T(1) / a.sw[k];
   }
   a.U = (const T*)U; a.V = (const T*)V; a.topg = (const T*)topg; a.thk = (const T*)thk; a.W = (T*)W;
   const int n_strips = (nx + kVfCols - 1) / kVfCols;

@@ -121,3 +121,15 @@ def test_unsupported_methods_raise():
     for over in [{"vert_flow": {"method": "twolayers"}}, {"vert_flow": {"version": 1}}]:
         with pytest.raises(NotImplementedError):
             vert_flow.update(default_cfg(over), st)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_weights_that_start_at_zero(dtype):
+    """The lowest layers of weight zero: their running mean 0 / 0 counts as 0, as
+    the layer of height zero needs it; level 0 is the same bits as with a weight."""
+    U, V, topg, thk, lv, w = _case(5, 40, 70, 3, dtype)
+    w0 = w.numpy()[:, 0, 0].copy()
+    w0[0] = 0
+    W = K.vertical_velocity(dev(U), dev(V), dev(topg), dev(thk), lv.numpy(), w0, 50.0)
+    ref = K.vertical_velocity(dev(U), dev(V), dev(topg), dev(thk), lv.numpy(), w.numpy()[:, 0, 0], 50.0)
+    assert bool(torch.isfinite(W).all()) and torch.equal(W[0], ref[0])
