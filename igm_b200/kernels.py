@@ -14,31 +14,54 @@ from . import _lib as L
 class Workspace:
     """Zero-filled scratch for the reducing kernels (they leave it zeroed).
 
-    One per device/stream; grown on demand.  Calls that share it must be
+    One per device and stream; grown on demand.  Calls that share it must be
     ordered on one stream."""
 
     def __init__(self):
-        self.buf = None
+        self.buf = self.captured = None
+        self.outgrown = []
 
     def get(self, grid: L.Grid, device) -> tuple[int, int]:
         need = int(L.lib().igm_workspace_size(C.byref(grid)))
         if need == 0:
             L.check(1, f"igm_workspace_size rejected grid {grid.batch}x{grid.nz}x{grid.ny}x{grid.nx}: "
                        + L.lib().igm_last_error().decode())
-        if self.buf is None or self.buf.numel() < need or (self.buf.device != device
-                                                           and self.buf.device != torch.device(device)):
-            self.buf = torch.zeros(max(need, 1 << 16), dtype=torch.uint8, device=device)
-        return self.buf.data_ptr(), self.buf.numel()
+        device = device if isinstance(device, torch.device) else torch.device(device)
+        if device.index is None:
+            device = torch.device(device.type, torch.cuda.current_device())
+        buf = self.buf
+        same = buf is not None and buf.device == device
+        if not same or buf.numel() < need:
+            # at least doubled, and what it replaces is kept: another thread on this stream may be about to launch
+            # with that one
+            buf = torch.zeros(max(need, 2 * buf.numel() if same else 1 << 16), dtype=torch.uint8, device=device)
+            if torch.cuda.is_current_stream_capturing():
+                self.captured = buf  # zero-filled when the graph runs, not now: for this launch alone
+            else:
+                if same:
+                    self.outgrown.append(self.buf)
+                self.buf = buf
+        return buf.data_ptr(), buf.numel()
 
 
+MAX_WORKSPACES = 64  # (device, stream) pairs; beyond it the one made first is dropped
 _WS: dict = {}
 
 
-def workspace(device) -> Workspace:
-    key = device if isinstance(device, torch.device) else torch.device(device)
-    if key not in _WS:
-        _WS[key] = Workspace()
-    return _WS[key]
+def workspace(device, stream=None) -> Workspace:
+    """The workspace of a device's stream (a raw pointer; default the current
+    stream).  Launches on two streams may run at the same time, so they share
+    none.  Keep the returned object until the launch: it owns the memory."""
+    key = (device if isinstance(device, torch.device) else torch.device(device),
+           L.stream_ptr() if stream is None else stream)
+    ws = _WS.get(key)
+    if ws is None:
+        ws = Workspace()
+        if not torch.cuda.is_current_stream_capturing():
+            while len(_WS) >= MAX_WORKSPACES:
+                _WS.pop(next(iter(_WS)), None)
+            ws = _WS.setdefault(key, ws)
+    return ws
 
 
 def fields_struct(thk, usurf, arrhenius, slidingco) -> L.Fields:
@@ -63,18 +86,20 @@ def energy(U, V, thk, usurf, arrhenius, slidingco, dx, dzeta, phys=None, grad=Fa
     terms = terms_out if terms_out is not None else torch.empty(3, dtype=torch.float64, device=U.device)
     dU = torch.empty_like(U) if grad else None
     dV = torch.empty_like(V) if grad else None
-    wp, wn = workspace(U.device).get(g, U.device)
+    st = L.stream_ptr()
+    ws = workspace(U.device, st)
+    wp, wn = ws.get(g, U.device)
     f = fields_struct(thk, usurf, arrhenius, slidingco)
     if grad and grad_out is not None:
         if grad_out.dtype != U.dtype or grad_out.numel() != 1:
             raise ValueError("energy: grad_out must be one value of U's dtype")
         rc = L.lib().igm_energy_backward(L.dtype_code(U.dtype), C.byref(g), C.byref(ph), C.byref(f), L.ptr(U), L.ptr(V),
                                          L.ptr(dU), L.ptr(dV), L.ptr(grad_out), float(grad_count), L.ptr(terms), wp, wn,
-                                         L.stream_ptr())
+                                         st)
         L.check(rc, "igm_energy_backward")
     else:
         rc = L.lib().igm_energy(L.dtype_code(U.dtype), C.byref(g), C.byref(ph), C.byref(f), L.ptr(U), L.ptr(V),
-                                L.ptr(dU), L.ptr(dV), float(grad_scale), L.ptr(terms), wp, wn, L.stream_ptr())
+                                L.ptr(dU), L.ptr(dV), float(grad_scale), L.ptr(terms), wp, wn, st)
         L.check(rc, "igm_energy")
     if squeeze and grad:
         dU, dV = dU[0], dV[0]

@@ -331,3 +331,72 @@ def test_backward_of_a_lazily_negated_gradient():
     got = torch.autograd.grad(iceflow_energy(U, V, *f, 100.0, dz), [U, V], grad_outputs=g)
     ref = torch.autograd.grad(iceflow_energy(U, V, *f, 100.0, dz), [U, V], grad_outputs=g.resolve_neg())
     assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
+
+
+def test_two_streams_share_no_workspace():
+    """Energies and gradients differentiated on two streams at once, without a
+    wait between them, against one after another; then one more on each, whose
+    scratch they must have left clean."""
+    from igm_b200.energy import iceflow_energy
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    sets, ref = [], []
+    for s, n in enumerate((190, 230)):
+        st = O.valley_glacier(n, n, 100.0, seed=s, varying_coeffs=True)
+        rng = np.random.default_rng(s)
+        f = [dev(st[k], torch.float32) for k in ["thk", "usurf", "arrhenius", "slidingco"]]
+        dz = O.compute_zeta_dzeta(O.compute_levels(6, 4.0))[1].numpy()
+        U, V = (dev(rng.normal(5, 9, (6, n, n)), torch.float32).requires_grad_(True) for _ in range(2))
+        sets.append((U, V, *f, 100.0, dz))
+        c = iceflow_energy(*sets[s])
+        ref.append((c.detach(), *torch.autograd.grad(c, [U, V])))
+    with torch.cuda.stream(streams[0]):
+        a = K.workspace(torch.device("cuda", 0))
+    with torch.cuda.stream(streams[1]):
+        b = K.workspace(torch.device("cuda", 0))
+    assert a is not b and a is K.workspace(torch.device("cuda", 0), streams[0].cuda_stream)
+    torch.cuda.synchronize()
+    got = [[], []]
+    for _ in range(25):
+        for s, stream in enumerate(streams):
+            with torch.cuda.stream(stream):
+                c = iceflow_energy(*sets[s])
+                got[s].append((c.detach(), *torch.autograd.grad(c, sets[s][:2])))
+    torch.cuda.synchronize()
+    for s in range(2):
+        for g in got[s]:
+            assert all(torch.equal(x, y) for x, y in zip(g, ref[s]))
+        with torch.cuda.stream(streams[s]):
+            assert torch.equal(iceflow_energy(*sets[s]).detach(), ref[s][0])
+    assert all(int(w.buf[:256].sum()) == 0 for w in (a, b))  # tickets and error word
+
+
+def test_workspaces_are_bounded():
+    dev0 = torch.device("cuda", 0)
+    made = [K.workspace(dev0, -1 - i) for i in range(K.MAX_WORKSPACES + 3)]  # keys of no stream: nothing is launched
+    assert len(K._WS) == K.MAX_WORKSPACES and K.workspace(dev0, -1) is not made[0]
+    for i in range(K.MAX_WORKSPACES + 3):
+        K._WS.pop((dev0, -1 - i), None)
+
+
+def test_captured_energies():
+    """Two graphs of an energy and its gradient, captured after a warm-up on
+    another stream, replayed in turn with other inputs before any eager call on
+    the capture's stream."""
+    ny, nx, nz = 90, 100, 5
+    st = O.valley_glacier(ny, nx, 100.0, seed=3, varying_coeffs=True)
+    f = [dev(st[k], torch.float32) for k in ["thk", "usurf", "arrhenius", "slidingco"]]
+    dz = O.compute_zeta_dzeta(O.compute_levels(nz, 4.0))[1].numpy()
+    U, V = (torch.zeros((nz, ny, nx), device="cuda") for _ in range(2))
+    K.energy(U, V, *f, 100.0, dz, grad=True)
+    graphs, outs = [], []
+    for _ in range(2):
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1]):
+            outs.append(K.energy(U, V, *f, 100.0, dz, grad=True))
+    rng = np.random.default_rng(4)
+    for g, out in list(zip(graphs, outs))[::-1] * 2:
+        U.copy_(torch.as_tensor(rng.normal(20, 10, U.shape)))
+        V.copy_(torch.as_tensor(rng.normal(0, 10, U.shape)))
+        g.replay()
+        ref = K.energy(U, V, *f, 100.0, dz, grad=True)
+        assert all(torch.equal(a, b) for a, b in zip(out, ref))
