@@ -1841,6 +1841,22 @@ extern "C" int igm_conv3x3_backward(int batch, int height, int width, const void
   return launch_status("conv3x3_bwd_kernel");
 }
 
+static bool stream_captured(cudaStream_t st) {
+  cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &c) != cudaSuccess) (void)cudaGetLastError();  // (the launch reports it)
+  return c != cudaStreamCaptureStatusNone;
+}
+
+// A captured launch is replayed with the epoch it was captured with, which the first replay leaves in every
+// flag: later ones would wait for nothing.  So the flags are cleared inside the graph, ahead of the launch.
+static int clear_captured_flags(int* flags, size_t n, cudaStream_t st) {
+  if (!stream_captured(st)) return IGM_OK;
+  const cudaError_t e = cudaMemsetAsync(flags, 0, n * sizeof(int), st);
+  if (e == cudaSuccess) return IGM_OK;
+  set_error("clearing the flags of a captured launch: %s", cudaGetErrorString(e));
+  return IGM_ERR_CUDA;
+}
+
 template <int R, int EPI>
 static int stack_launch(int batch, int height, int width, int nlayers, const void* x, void* const* outs,
                         const void* const* wpacks, const float* const* biases, const void* const* masks, int* flags,
@@ -1878,7 +1894,7 @@ static int stack_launch(int batch, int height, int width, int nlayers, const voi
   a.err = err;
   static bool configured = false;
   int rc = set_smem(conv3x3_stack_kernel<R, EPI>, SMEM, &configured);
-  if (rc) return rc;
+  if (rc || (rc = clear_captured_flags(flags, (size_t)nlayers * a.n_tiles, as_stream(stream)))) return rc;
   const int grid = a.n_tiles < sm_count() ? a.n_tiles : sm_count();
   // cooperative: every CTA resident at once, which the inter-CTA tile flags rely on
   cudaLaunchConfig_t cfg = {};
@@ -1943,10 +1959,8 @@ extern "C" int igm_conv3x3_stack_dgrad(int batch, int height, int width, int nla
   IGM_CHECK_ARG(batch >= 1 && height >= 1 && width >= 1 && batch <= 65535, IGM_ERR_BAD_SHAPE,
                 "igm_conv3x3_stack_dgrad: bad shape %dx%dx%d", batch, height, width);
   const size_t tiles = (size_t)batch * ((width + kTW - 1) / kTW) * ((height + kRows - 1) / kRows);
-  // A captured launch would be replayed with the same epoch, its flags already up; the layers need none.
-  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-  cudaStreamIsCapturing(as_stream(stream), &capture);
-  if (tiles > 8 * (size_t)sm_count() || capture != cudaStreamCaptureStatusNone) {
+  // (Captured, the layers need no clearing of the flags.)
+  if (tiles > 8 * (size_t)sm_count() || stream_captured(as_stream(stream))) {
     IGM_CHECK_ARG(nlayers >= 1 && nlayers <= kStackMax && outs && wpacks && masks, IGM_ERR_BAD_ARGUMENT,
                   "igm_conv3x3_stack_dgrad: NULL argument, or not 1 .. %d layers", kStackMax);
     for (int k = 0; k < nlayers; ++k) {
@@ -2005,7 +2019,8 @@ extern "C" int igm_conv3x3_chain(int batch, int height, int width, int nlayers, 
   a.err = err;
   static bool configured = false;
   int rc = set_smem(conv3x3_chain_kernel, G::SMEM, &configured);
-  if (rc) return rc;
+  if (rc || (rc = clear_captured_flags(flags, igm_conv3x3_chain_flags_len(batch, height, width, nlayers), as_stream(stream))))
+    return rc;
   const long long rows = (long long)batch * a.strips * height;
   const int grid = (int)(rows < sm_count() ? rows : sm_count());
   // cooperative: every CTA resident at once, which the row flags rely on

@@ -539,7 +539,9 @@ IGM_API int igm_conv1x1_wgrad(int batch, int height, int width, const void* x, c
  * read are stored (a cooperative launch with per-tile flags).  flags: a device
  * int buffer of igm_conv3x3_stack_flags_len ints holding no value equal to
  * epoch (a zeroed buffer and a per-call counter from 1 serve).  outs, wpacks,
- * biases: host arrays of nlayers device pointers. */
+ * biases: host arrays of nlayers device pointers.  Under stream capture the
+ * clearing of the flags is captured ahead of the launch, so a graph may be
+ * replayed, and eager calls on the same flags may come between. */
 IGM_API int igm_conv3x3_stack(int batch, int height, int width, int nlayers, const void* x, void* const* outs,
                               const void* const* wpacks, const float* const* biases, int* flags, int epoch,
                               float alpha, int* err, void* stream);
@@ -560,7 +562,7 @@ IGM_API int igm_conv3x3_stack_dgrad(int batch, int height, int width, int nlayer
  * gets layer 2k + 1's output, mids[k] (may be NULL) layer 2k's.  outs may
  * alternate between two buffers, neither of them x.  flags: device int buffer of
  * igm_conv3x3_chain_flags_len ints holding no value equal to epoch (non-zero); the call
- * leaves it filled with epoch.  height >= 8.  The same bits as nlayers igm_conv3x3 calls; for
+ * leaves it filled with epoch; under capture as igm_conv3x3_stack.  height >= 8.  The same bits as nlayers igm_conv3x3 calls; for
  * grids that give every SM some rows (the caller's choice). */
 IGM_API int igm_conv3x3_chain(int batch, int height, int width, int nlayers, int cin_first, const void* x,
                               void* const* mids, void* const* outs, const void* const* wpacks,

@@ -465,3 +465,40 @@ def test_conv_stack_dgrad_captured():
         graph.replay()
         torch.cuda.synchronize()
         assert int(err.item()) == 0 and torch.equal(two[0], ref)
+
+
+@pytest.mark.parametrize("H,W,nl,chain", [(100, 100, 5, False), (300, 400, 4, False), (840, 1000, 5, True)])
+def test_forward_captured(H, W, nl, chain):
+    """A graph of the network's forward, on the stack's and the chain's path,
+    replayed with other inputs each time and with eager calls between, whose
+    epochs and flags it shares: the bits of the eager forward."""
+    from igm_b200.cnn import CNN
+    net = CNN(nb_layers=nl, cin=5, nout=8, init="he_normal", seed=1, scales=[1 / 300, 1 / 3000, 0.01, 10, 0.01])
+    buf = net.buffers(1, H, W, train=False)
+    assert buf["chain"] == chain
+    g = torch.Generator(device="cuda").manual_seed(2)
+    f = [torch.empty(H, W, device="cuda") for _ in range(4)]
+
+    def forward():
+        net.prepare_input(f, 50.0, [(0, 0)], H, W, buf)
+        return net.forward(buf, 1, H, W, thk_mask=f[0])
+
+    def draw():
+        for t, scale in zip(f, (300.0, 3000.0, 100.0, 0.1)):
+            t.copy_(torch.rand(H, W, generator=g, device="cuda") * scale)
+
+    draw()
+    forward()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        U, V = forward()
+    for k in range(4):
+        draw()
+        graph.replay()
+        got = U.clone(), V.clone()
+        if k != 1:  # (once, two replays in a row)
+            U.zero_(), V.zero_()
+            ref = [t.clone() for t in forward()]
+            assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
+    net.check_errors()
