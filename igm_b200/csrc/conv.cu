@@ -1958,11 +1958,14 @@ extern "C" int igm_conv3x3_stack_dgrad(int batch, int height, int width, int nla
   // and 215, 1000 x 1000 569 and 556, 2048 x 2048 1995 and 2212: they cross at 8 tiles of 8 rows per SM.
   IGM_CHECK_ARG(batch >= 1 && height >= 1 && width >= 1 && batch <= 65535, IGM_ERR_BAD_SHAPE,
                 "igm_conv3x3_stack_dgrad: bad shape %dx%dx%d", batch, height, width);
+  IGM_CHECK_ARG(nlayers >= 1 && nlayers <= kStackMax && g && outs && wpacks && masks, IGM_ERR_BAD_ARGUMENT,
+                "igm_conv3x3_stack_dgrad: NULL argument, or not 1 .. %d layers", kStackMax);
+  for (int k = 0; k < nlayers; ++k)
+    IGM_CHECK_ARG(outs[k] != (k ? outs[k - 1] : g), IGM_ERR_BAD_ARGUMENT,
+                  "igm_conv3x3_stack_dgrad: layer %d: the output aliases the layer's input", k);
   const size_t tiles = (size_t)batch * ((width + kTW - 1) / kTW) * ((height + kRows - 1) / kRows);
   // (Captured, the layers need no clearing of the flags.)
   if (tiles > 8 * (size_t)sm_count() || stream_captured(as_stream(stream))) {
-    IGM_CHECK_ARG(nlayers >= 1 && nlayers <= kStackMax && outs && wpacks && masks, IGM_ERR_BAD_ARGUMENT,
-                  "igm_conv3x3_stack_dgrad: NULL argument, or not 1 .. %d layers", kStackMax);
     for (int k = 0; k < nlayers; ++k) {
       const int rc = igm_conv3x3(IGM_CONV_DGRAD, batch, height, width, kCout, k ? outs[k - 1] : g, wpacks[k], nullptr,
                                  masks[k], outs[k], nullptr, 0, alpha, err, stream);

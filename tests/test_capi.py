@@ -133,3 +133,14 @@ def test_emulator_entries_validate_without_gpu(lib):
     empty = (C.c_size_t * 3)(0, 10, 10)
     rc = lib.igm_adam_clipnorm(2, empty, 16, 16, 16, 16, 16, 1e-3, 0.9, 0.999, 1e-7, 1.0, 1, None)
     assert rc == 2 and b"empty variable" in lib.igm_last_error()
+
+
+def test_dgrad_stack_refuses_an_output_on_its_input(lib):
+    """A layer's rows are read while others are written; checked before any CUDA call."""
+    def rc(g, *outs):
+        n = len(outs)
+        arr = lambda *v: (C.c_void_p * n)(*v)  # noqa: E731
+        return lib.igm_conv3x3_stack_dgrad(1, 16, 16, n, g, arr(*outs), arr(*[4096] * n), arr(*[8192] * n), 1024, 1, 0.01, None,
+                                           None)
+    for g, outs in ((16384, (16384,)), (16384, (32768, 32768)), (16384, (32768, 16384, 16384))):
+        assert rc(g, *outs) == 2 and b"alias" in lib.igm_last_error()
