@@ -1111,10 +1111,16 @@ __global__ void __launch_bounds__(kChThreads, 1) conv3x3_chain_kernel(const Chai
             }
           }
           if (!layer_a && ((j & 3) == 3 || j == rows - 1)) {
-            // a group of rows is stored: the publisher's turn when all eight warps say so
+            // a group of rows is stored: the publisher's turn when all eight warps say so (its barriers' phases
+            // allow it to be kChPub groups behind)
             tc::fence_proxy_async_global();
             __syncwarp();
             for (uint32_t n = 0; g >= *published + kChPub && n < (1u << 22) && !*gave_up; ++n) __nanosleep(20);
+            if (!(ok = (bool)__all_sync(0xffffffffu, g < *published + kChPub))) {
+              if (lane == 0 && !*gave_up) set_err(a.err, 50);
+              *gave_up = 1;
+              break;
+            }
             if (lane == 0) tc::mbar_arrive(&stored[g % kChPub]);
             ++g;
           }
