@@ -458,6 +458,7 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_stack_kernel(const
   if (warp == 0) {
     // ---------------- producer ----------------
     int it = 0;
+    int start = 0;  // the previous layer's first iteration
     bool ok = true;
     for (int k = 0; k < a.nlayers && ok; ++k) {
       const __nv_bfloat16* src = k == 0 ? a.in : a.out[k - 1];
@@ -469,11 +470,21 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_stack_kernel(const
           break;
         }
         unsigned char* st = smem + s * G::STAGE;
-        if (t == first(k) && lane == 0) {
-          // this layer's weights, on the barrier of its first tile (their buffer's last reader, layer
-          // k - 2, completed: the commit that released this stage covers every earlier MMA)
-          tc::mbar_expect_tx_only(&full[s], G::WBYTES);
-          tc::bulk_load(smem + G::OFF_W + (k & 1) * G::WBYTES, a.wpack[k], G::WBYTES, &full[s]);
+        if (t == first(k)) {
+          // this layer's weights, on the barrier of its first tile.  Their buffer's last reader, layer k - 2,
+          // has completed: its last iteration is start - 1, and the commit that released this stage covers
+          // the iterations up to it - NST, with two stages always that one (layer k - 1 has a tile here)
+          const int last = start - 1;
+          if (NST > 2 && k >= 2 && last > it - NST && !tc::mbar_wait(&empty[last % NST], (last / NST) & 1)) {
+            if (lane == 0) set_err(a.err, 31);
+            ok = false;
+            break;
+          }
+          start = it;
+          if (lane == 0) {
+            tc::mbar_expect_tx_only(&full[s], G::WBYTES);
+            tc::bulk_load(smem + G::OFF_W + (k & 1) * G::WBYTES, a.wpack[k], G::WBYTES, &full[s]);
+          }
         }
         __syncwarp();
         const int txi = t % a.tiles_w, rest = t / a.tiles_w;
