@@ -516,6 +516,8 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_stack_kernel(const
         load_tile<true>(src, a.H, a.W, 4, b, tyi * R - 1, R + 2, txi * kTW - 1, kBoxW, st, &full[s], lane);
       }
     }
+    if (!ok)  // let the copies in flight end (a layer's weights leave before the wait for its flags)
+      for (int i = 0; i < 1000; ++i) __nanosleep(1000);
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     if (lane == 0) {
