@@ -1293,7 +1293,8 @@ static int head_fwd_mma(int batch, int h, int w, const void* act, const float* h
   const long long chunks = (long long)batch * h * ((w + 31) / 32), blocks = (chunks + kHmWarps - 1) / kHmWarps;
   IGM_CHECK_ARG(chunks < (1ll << 30) && ((uintptr_t)act & 15) == 0, IGM_ERR_BAD_SHAPE,
                 "igm_cnn_head_inference: more than 2^30 runs of 32 pixels, or an activation not 16-byte aligned");
-  const int grid = (int)(blocks < 148 * 2 ? blocks : 148 * 2);  // resident at once: a warp splits the weights once
+  const int cap = 2 * igm_conv_sm_count();  // two CTAs per SM, resident at once: a warp splits the weights once
+  const int grid = (int)(blocks < cap ? blocks : cap);
   constexpr size_t smem = sizeof(HeadMmaSmem<(2 * NZ + 7) / 8>);
   static bool configured = false;
   if (!configured) {
