@@ -502,3 +502,34 @@ def test_forward_captured(H, W, nl, chain):
             ref = [t.clone() for t in forward()]
             assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
     net.check_errors()
+
+
+@pytest.mark.parametrize("B,H,W,nz", [(1, 4, 128, 1), (2, 9, 173, 4), (1, 5, 31, 5), (1, 33, 100, 10), (3, 2, 33, 16)])
+@pytest.mark.parametrize("masked", [False, True])
+def test_head_inference_with_fp32_weights(B, H, W, nz, masked):
+    """The inference head without derived velocities, weights with all three of
+    their bf16 parts non-zero: within 1e-5 of the output's scale of a float64
+    evaluation, as with one part, and no further off than twice what the FP32
+    chains of igm_cnn_head_forward are.  (Without the third part an output is
+    off by 4e-7 of its scale on average, without the second by 3e-4; chains 2e-8.)"""
+    g = torch.Generator().manual_seed(B + H + W + nz)
+    lib, st = L.lib(), L.stream_ptr()
+    a32 = bf(torch.randn(B, 32, H, W, generator=g))
+    act = to_rc(a32).to(torch.bfloat16).cuda()
+    wh = torch.randn(32, 2 * nz, generator=g).cuda()
+    parts = wh.clone()
+    for _ in range(2):
+        parts = parts - parts.to(torch.bfloat16).float()
+    assert float((parts != 0).float().mean()) > 0.9
+    bh, thk = (torch.randn(2 * nz, generator=g) * 0.1).cuda(), (torch.rand(B, H, W, generator=g) - 0.3).cuda()
+    err = []
+    y = (torch.einsum("bchw,cj->bjhw", a32.double(), wh.cpu().double()) + bh.cpu().double()[None, :, None, None]) * 2.5
+    y = torch.where((thk.cpu() > 0)[:, None], y, torch.zeros_like(y)) if masked else y
+    for chains in (False, True):
+        U, V = (torch.full((B, nz, H, W), 7.0, device="cuda") for _ in range(2))
+        args = (B, H, W, nz, act.data_ptr(), wh.data_ptr(), bh.data_ptr(), 2.5, U.data_ptr(), V.data_ptr(),
+                thk.data_ptr() if masked else None)
+        L.check(lib.igm_cnn_head_forward(*args, st) if chains else lib.igm_cnn_head_inference(*args, None, *[None] * 7, st))
+        err.append((torch.cat([U, V], 1).cpu().double() - y).abs() / y.abs().max())
+    assert float(err[0].max()) <= 1e-5
+    assert float(err[0].square().mean().sqrt()) <= 2 * float(err[1].square().mean().sqrt())
