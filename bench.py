@@ -527,6 +527,8 @@ def run_ours(args, rank, world, dist):
     clocks = clk.stop()
     launches = lib.igm_launch_count() - l0
     st.iceflow_model.event_hook = None
+    net = st.iceflow_model
+    res["conv_path"] = dict(layers=net.L, chain=net.buffers(1, *st.thk.shape, train=False)["chain"])
     years_e = float(st.t) - t_start
     el_e = max_over_ranks(el_e)
     res["emulated"] = dict(years=years_e, seconds=el_e, years_per_s=years_e / el_e)
@@ -809,32 +811,42 @@ def assimilation_cpu(args, crop):
             "sample": f"one optimize_update iteration of the oracle on a {crop}x{crop} crop (second of two), "
                       f"scaled by ({args.size}/{crop})^2; emulator retraining not included"}
 
-def roofline_conv(conv_ms, size, peaks, layers=16):
-    """The forward convolutions of an inference in one launch (the chain: the
-    first layer, 16-channel split input, and 15 layers of 32 -> 32 channels, two
-    per pass over memory): multiplications and additions of the 3x3 taps
-    against the measured bf16 rate; algorithmic bytes = per pass one read of its
-    input (32 B per pixel for the first, then 64) and one write of 64 B."""
+def roofline_conv(conv_ms, size, peaks, layers=16, chain=True):
+    """The forward convolutions of an inference that CNN.event_hook timed, of a
+    network of ``layers`` 3x3 layers.  ``chain``: all of an even number of layers
+    in one launch, two per pass over memory; multiplications and additions of the
+    3x3 taps (5 input fields in the first layer, whose 16 channels are split copies
+    of them) against the measured bf16 rate; algorithmic bytes = per pass one read
+    of its input (32 B per pixel for the first, then 64) and one write of 64 B.
+    Else the 32 -> 32 channel layers behind the first in one launch, a read and a
+    write of 64 B per pixel each, against the measured copy rate."""
     if not conv_ms:
         return None
     t = float(np.mean(conv_ms)) / 1e3
-    byts = (layers // 2 * 128 - 32) * size * size
-    achieved = 2 * 9 * 32 * (16 + 32 * (layers - 1)) * size * size / t / 1e12
-    peak = peaks.get("bf16_tflops", 1590.0)
-    # DRAM traffic of one launch from the committed ncu capture of the same launch (16 layers,
+    layers = layers // 2 * 2 if chain else layers - 1
+    byts = (layers * 64 - 32 if chain else layers * 2 * 64) * size * size
+    # DRAM traffic of one launch from the committed ncu capture of the same launch (16 or 15 layers,
     # batch 1 x 1000 x 1000), scaled to this launch's pixels
     traffic = None
-    prof = os.path.join(ROOT, "profiles", "conv3x3_chain_16x1000x1000.txt")
+    prof = os.path.join(ROOT, "profiles", f"conv3x3_{'chain' if chain else 'stack'}_{layers}x1000x1000.txt")
     if os.path.exists(prof):
         for line in open(prof):
             if line.startswith("dram_bytes_per_launch:"):
                 traffic = round(float(line.split(":")[1]) * (size * size) / (1000 * 1000))
-    return {"kernel": f"conv3x3_chain_kernel (tcgen05, {layers} layers per launch, two per pass over memory)",
-            "bound": "tensor",
-            "achieved": round(achieved, 1), "peak": peak, "unit": "TFLOP/s", "frac": round(achieved / peak, 4),
-            "traffic": traffic, "algorithmic_bytes": byts, "avg_launch_us": round(t * 1e6, 2),
-            "avg_layer_us": round(t * 1e6 / layers, 2), "launches": len(conv_ms),
-            "peak_source": "MEASURED_PEAKS.json bf16_tflops (of measured)" if "bf16_tflops" in peaks else "fallback"}
+    out = {"kernel": f"conv3x3_chain_kernel (tcgen05, {layers} layers per launch, two per pass over memory)" if chain
+           else f"conv3x3_stack_kernel (tcgen05, {layers} layers of cin 32 per launch)"}
+    if chain:
+        achieved, peak = 2 * 9 * 32 * (5 + 32 * (layers - 1)) * size * size / t / 1e12, peaks.get("bf16_tflops", 1590.0)
+        out.update(bound="tensor", unit="TFLOP/s", peak_source="MEASURED_PEAKS.json bf16_tflops (of measured)"
+                   if "bf16_tflops" in peaks else "fallback")
+    else:
+        achieved, peak = byts / t / 1e9, peaks.get("hbm_gbs", 6650.0)
+        out.update(bound="hbm", unit="GB/s", peak_source="MEASURED_PEAKS.json hbm_gbs (of measured)"
+                   if "hbm_gbs" in peaks else "fallback")
+    out.update(achieved=round(achieved, 1), peak=peak, frac=round(achieved / peak, 4), traffic=traffic,
+               algorithmic_bytes=byts, avg_launch_us=round(t * 1e6, 2), avg_layer_us=round(t * 1e6 / layers, 2),
+               launches=len(conv_ms))
+    return out
 
 
 def plain_run_100x100(args, cpu_steps=2, gpu_max_steps=3000, gpu_max_s=40.0):
@@ -1301,7 +1313,7 @@ def main():
             "fallback_checks": res["fallback_checks"], "fallbacks": res["fallbacks"],
             "years_per_time_step_emulated": em["years"] / (K * TIME_STEPS_PER_STEP),
             "years_per_time_step_plain": sv["years"] / (K * TIME_STEPS_PER_STEP),
-            "roofline": roofline_conv(conv_ms, args.size, peaks),
+            "roofline": roofline_conv(conv_ms, args.size, peaks, **res["conv_path"]),
             "clocks": clocks, "gpu_launches": int(launches), "e2e": e2e}
     if rank == 0:
         if "plain_100x100" in det:
