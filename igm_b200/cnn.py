@@ -63,8 +63,10 @@ class CNN:
         self.wpack_b = torch.zeros(max(self.L - 1, 1) * 9 * 4 * F * 8, dtype=torch.bfloat16, device=self.device)
         self.init_weights(init, seed)
         self._bufs = {}
-        self.event_hook = None  # list: (start, end) CUDA events of each inference's 32-channel conv stack
-        self._epoch = 0  # tile-flag epoch of the conv stack launches
+        # list: (start, end) CUDA events of each inference's launch of many layers: the chain (buffers' "chain"), with
+        # the first layer in it, or the 32-channel stack behind the first layer
+        self.event_hook = None
+        self._epoch = 0  # flag epoch of the stack and chain launches
         self.err = torch.zeros(1, dtype=torch.int32, device=self.device)
         self.n_sm = int(lib.igm_conv_sm_count())
 
@@ -112,9 +114,6 @@ class CNN:
     def _wf(self, l):
         off = 0 if l == 0 else 9 * 2 * F * 8 + (l - 1) * 9 * 4 * F * 8
         return self.wpack_f.data_ptr() + 2 * off
-
-    def _wb(self, l):
-        return self.wpack_b.data_ptr() + 2 * (l - 1) * 9 * 4 * F * 8
 
     def _b(self, l):
         return self.params.data_ptr() + 4 * self.offsets[2 * l + 1]
@@ -173,14 +172,14 @@ class CNN:
         B = len(windows)
         y0 = (C.c_int * B)(*[int(a) for a, _ in windows])
         x0 = (C.c_int * B)(*[int(b) for _, b in windows])
-        sc = (C.c_float * 5)(*self.scales.tolist())
+        sc = self._scales()
         rc = L.lib().igm_cnn_input(B, h, w, ny, nx, *[_p(f) for f in fields_full], float(dx), sc, y0, x0,
                                    _p(buf["X"]), *[_p(f) for f in buf["fields"]], L.stream_ptr())
         L.check(rc, "igm_cnn_input")
         buf["dx"] = float(dx)
 
     def _scales(self):
-        return (C.c_float * 5)(*[float(s) for s in self.scales])
+        return (C.c_float * 5)(*map(float, self.scales))  # (any sequence: a caller may have set it)
 
     def forward(self, buf, B, h, w, thk_mask=None, keep_acts=False, vert_weight=None):
         """Runs the network on the windowed fields of ``buf`` (prepare_input):

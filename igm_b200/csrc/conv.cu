@@ -672,7 +672,7 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_stack_kernel(const
 // ---------------------------------------------------------------------------
 // forward of a chain of layers, two layers per pass over memory
 // ---------------------------------------------------------------------------
-// A layer alone reads and writes 64 B per pixel and multiplies 18,432 times:
+// A layer alone reads and writes 64 B and multiplies and adds 9,216 times per pixel:
 // run one by one the layers move more bytes between the SMs and memory than the
 // tensor cores take time for (26 us per 1000 x 1000 layer against 11 us of
 // math).  Here a pass over memory computes two layers (A, then B): a CTA walks

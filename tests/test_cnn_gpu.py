@@ -256,3 +256,15 @@ def test_two_layers_per_pass_gives_the_same_bits(nl, keep):
     if keep:
         assert all(torch.equal(a, b) for a, b in zip(acts, buf["acts"]))
     assert flags.numel() == (nl // 2) * 8 * h
+
+
+def test_scales_may_be_any_sequence():
+    f = [torch.rand(9, 12, device="cuda") for _ in range(4)]
+    X = []
+    for scales in (np.array([0.1, 0.2, 0.3, 0.4, 0.5], np.float32), [0.1, 0.2, 0.3, 0.4, 0.5]):
+        net = CNN(nb_layers=2, cin=5, nout=4)
+        net.scales = scales
+        buf = net.buffers(1, 9, 12, train=False)
+        net.prepare_input(f, 50.0, [(0, 0)], 9, 12, buf)
+        X.append(buf["X"].clone())
+    assert torch.equal(*X)
