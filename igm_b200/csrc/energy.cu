@@ -136,11 +136,15 @@ template <> __device__ __forceinline__ Two<float> rcbrt2<float>(Two<float> x) {
 // ice every node's gradient and moments are zero, which the square root and the
 // division would each take their slow paths for: an iteration at 1000 x 1000 x
 // 10, half of it ice, 173.5 -> 146 us, at 100 x 100 25.9 -> 22.1.
+// FP32 with other copies than TMA's divides all the same (ZERO false): there ice
+// everywhere paid more for the test than bare ground gained, 701 x 1003 x 10 with
+// and without it 155 and 130 us, half ice 148 and 150; 2000 x 2001 795 and 680,
+// 764 and 775.
 // With epsilon 0 that step is 0 / 0, not zero: such a solve takes the element
-// copies' variant, the only one that looks at epsilon (ANY_EPS; in the others
-// the look took 1 % of an iteration).
-template <typename T, bool ANY_EPS> __device__ __forceinline__ T adam_step(T m_alpha, T v, T eps) {
-  return m_alpha == T(0) && (!ANY_EPS || eps > T(0)) ? T(0) : m_alpha / (Math<T>::sqrt(v) + eps);
+// copies' variant, which divides in FP32 and is the only one that looks at epsilon
+// in FP64 (ANY_EPS; in the others the look took 1 % of an iteration).
+template <typename T, bool ZERO, bool ANY_EPS> __device__ __forceinline__ T adam_step(T m_alpha, T v, T eps) {
+  return ZERO && m_alpha == T(0) && (!ANY_EPS || eps > T(0)) ? T(0) : m_alpha / (Math<T>::sqrt(v) + eps);
 }
 
 enum StencilMode { kEnergyOnly = 0, kGradient = 1, kAdamStep = 2 };
@@ -276,6 +280,7 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
   // bare ground can: with the skip half ice at 1000 x 1000 x 10 is 147 us either way and all ice 163 us, without it
   // 153.  FP64 there: half ice 290 us with it and 324 without, all ice 351 and 348.
   constexpr bool kSkip = STD && (MODE != kAdamStep || sizeof(T) == 8);
+  constexpr bool kZeroSteps = LOAD == kLoadTma || sizeof(T) == 8;  // adam_step
   const bool glen3 = STD || a.glen3, weert3 = STD || a.weert3, fnge = !STD && a.fnge;
   constexpr int TYC = 2 * TYP;  // cell rows per tile
   constexpr int NT = kCW * TYP;
@@ -680,14 +685,14 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
           v += (gu * gu - v) * b2c;
           a.mU[o] = m;
           a.vU[o] = v;
-          Unxt[o] = SM.N[st][0][sm] - adam_step<T, LOAD == kLoadElems>(m * alpha, v, a.eps);
+          Unxt[o] = SM.N[st][0][sm] - adam_step<T, kZeroSteps, LOAD == kLoadElems>(m * alpha, v, a.eps);
           m = SM.M[st][1][sm];
           v = SM.M[st][3][sm];
           m += (gv - m) * b1c;
           v += (gv * gv - v) * b2c;
           a.mV[o] = m;
           a.vV[o] = v;
-          Vnxt[o] = SM.N[st][1][sm] - adam_step<T, LOAD == kLoadElems>(m * alpha, v, a.eps);
+          Vnxt[o] = SM.N[st][1][sm] - adam_step<T, kZeroSteps, LOAD == kLoadElems>(m * alpha, v, a.eps);
         }
       }
     };
