@@ -242,6 +242,7 @@ struct StencilSmem {
   uint64_t full[kStages];                       // TMA arrival of a level
   uint64_t ffull[2];                            // TMA arrival of a tile's 2-D fields
   unsigned int ticket;
+  T grad_scale;
 };
 
 // Thread rows per CTA (each thread row = one warp = two cell rows).
@@ -480,7 +481,9 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
 #pragma unroll 1
   for (int q = 0; q < kAhead; ++q) issue_next();
 
-  const T gscale = MODE == kGradient && a.grad_out ? (T)((double)__ldg(a.grad_out) / a.grad_count) : a.grad_scale;
+  // (visible with the first tile's fields; here since a register more spills in the general physics' variant)
+  if (MODE == kGradient && tid == 0)
+    SM.grad_scale = a.grad_out ? (T)((double)__ldg(a.grad_out) / a.grad_count) : a.grad_scale;
   const T half = T(0.5), quarter = T(0.25);
   const P H = two(half), Q4 = two(quarter), zero = two(T(0));
   const P HI = two(half * a.inv_dx);
@@ -595,7 +598,7 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
     const P egc = thks * two(a.Kg * T(0.125));
     // adjoint constants (grad_scale folded in; zero for cells outside the domain, whose
     // contributions then vanish without masking)
-    const P okm = sel(cok[0], cok[1], two(gscale), zero);
+    const P okm = sel(cok[0], cok[1], two(MODE == kGradient ? SM.grad_scale : a.grad_scale), zero);
     const P gshc = esc * okm;                // dE/d(bq sr2w) per unit dzeta
     const P gxc = egc * ssx * okm, gyc = egc * ssy * okm;  // dE/dS, dE/dSV per unit gravity weight
     const P csg = cs * okm * Q4;             // sliding: dE/dS = csg N^(s/2-1) (Us + tb sbx)
