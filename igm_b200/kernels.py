@@ -26,12 +26,12 @@ class Workspace:
         if need == 0:
             L.check(1, f"igm_workspace_size rejected grid {grid.batch}x{grid.nz}x{grid.ny}x{grid.nx}: "
                        + L.lib().igm_last_error().decode())
-        device = device if isinstance(device, torch.device) else torch.device(device)
-        if device.index is None:
-            device = torch.device(device.type, torch.cuda.current_device())
         buf = self.buf
-        same = buf is not None and buf.device == device
-        if not same or buf.numel() < need:
+        if buf is None or buf.numel() < need or buf.device != device:
+            device = _indexed(device)
+            same = buf is not None and buf.device == device
+            if same and buf.numel() >= need:
+                return buf.data_ptr(), buf.numel()
             # at least doubled, and what it replaces is kept: another thread on this stream may be about to launch
             # with that one
             buf = torch.zeros(max(need, 2 * buf.numel() if same else 1 << 16), dtype=torch.uint8, device=device)
@@ -44,6 +44,11 @@ class Workspace:
         return buf.data_ptr(), buf.numel()
 
 
+def _indexed(device) -> torch.device:
+    device = torch.device(device)
+    return device if device.index is not None else torch.device(device.type, torch.cuda.current_device())
+
+
 MAX_WORKSPACES = 64  # (device, stream) pairs; beyond it the one made first is dropped
 _WS: dict = {}
 
@@ -52,8 +57,9 @@ def workspace(device, stream=None) -> Workspace:
     """The workspace of a device's stream (a raw pointer; default the current
     stream).  Launches on two streams may run at the same time, so they share
     none.  Keep the returned object until the launch: it owns the memory."""
-    key = (device if isinstance(device, torch.device) else torch.device(device),
-           L.stream_ptr() if stream is None else stream)
+    if not isinstance(device, torch.device) or device.index is None:
+        device = _indexed(device)
+    key = (device, L.stream_ptr() if stream is None else stream)
     ws = _WS.get(key)
     if ws is None:
         ws = Workspace()
