@@ -509,6 +509,8 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_stack_kernel(const
           if (!__all_sync(0xffffffffu, got)) {
             if (lane == 0) set_err(a.err, 32);
             ok = false;
+#pragma unroll 1
+            for (int i = 0; i < 1000; ++i) __nanosleep(1000);  // a layer's weights may be in flight: let them land
             break;
           }
           tc::fence_proxy_async_global();  // the acquired data is read next by the bulk-copy (async) proxy
@@ -516,8 +518,6 @@ __global__ void __launch_bounds__(kConvFwdThreads, 1) conv3x3_stack_kernel(const
         load_tile<true>(src, a.H, a.W, 4, b, tyi * R - 1, R + 2, txi * kTW - 1, kBoxW, st, &full[s], lane);
       }
     }
-    if (!ok)  // let the copies in flight end (a layer's weights leave before the wait for its flags)
-      for (int i = 0; i < 1000; ++i) __nanosleep(1000);
   } else if (warp == 1) {
     // ---------------- MMA issuer ----------------
     if (lane == 0) {
