@@ -179,7 +179,7 @@ class CNN:
         buf["dx"] = float(dx)
 
     def _scales(self):
-        return (C.c_float * 5)(*map(float, self.scales))  # (any sequence: a caller may have set it)
+        return (C.c_float * 5)(*np.asarray(self.scales, np.float32).tolist())  # (a caller may have set another sequence)
 
     def forward(self, buf, B, h, w, thk_mask=None, keep_acts=False, vert_weight=None):
         """Runs the network on the windowed fields of ``buf`` (prepare_input):
