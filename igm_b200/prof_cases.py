@@ -2,7 +2,8 @@
 (``python -m igm_b200.prof_cases``; run it under ncu with -k and -c).
 
 Stencil (energy, energy + adjoint, one fused Adam iteration), transport and
-the vertical velocity at 1500 x 1500 x Nz 10 in FP32; the data-assimilation
+the vertical velocity at 1500 x 1500 x Nz 10 in FP32, the stencil's energy +
+adjoint at 1500 x 1501 too (row copies instead of TMA); the data-assimilation
 cost/gradient, flow direction and upwind divergence at 1500 x 1500 in FP32;
 the tensor-core convolution (forward, dgrad, wgrad, the fused backward) at
 batch 2 x 1000 x 1000 x 32 channels, and at batch 1 the forward and the
@@ -74,6 +75,10 @@ def main():
     K.vertical_velocity(U, V, topg, f[0], compute_levels(nz, 4.0), define_vertical_weight(nz, 4.0), 50.0,
                         method="incompressibility")
     assimilation(N, f, U[-1].contiguous(), V[-1].contiguous())
+    st = valley_glacier(N, N + 1, 50.0, seed=0, varying_coeffs=True)
+    U, V = (torch.as_tensor(rng.normal(m, 20, (nz, N, N + 1)).astype(np.float32)).cuda() for m in (30, 0))
+    K.energy(U, V, *[torch.as_tensor(st[k]).cuda() for k in ["thk", "usurf", "arrhenius", "slidingco"]], 50.0, dz,
+             grad=True)                                           # stencil: energy + adjoint, rows off 16 bytes
     B, H, W = 2, 1000, 1000                                       # 2 x 64 MB activations (> L2)
     x = torch.randn(B, H, 4, W, 8, device="cuda").to(torch.bfloat16)
     y = torch.empty_like(x)
