@@ -92,10 +92,10 @@ def energy(U, V, thk, usurf, arrhenius, slidingco, dx, dzeta, phys=None, grad=Fa
     terms = terms_out if terms_out is not None else torch.empty(3, dtype=torch.float64, device=U.device)
     dU = torch.empty_like(U) if grad else None
     dV = torch.empty_like(V) if grad else None
+    f = fields_struct(thk, usurf, arrhenius, slidingco)  # (refuses tensors that are not on the device)
     st = L.stream_ptr()
     ws = workspace(U.device, st)
     wp, wn = ws.get(g, U.device)
-    f = fields_struct(thk, usurf, arrhenius, slidingco)
     if grad and grad_out is not None:
         if grad_out.dtype != U.dtype or grad_out.numel() != 1:
             raise ValueError("energy: grad_out must be one value of U's dtype")

@@ -52,10 +52,10 @@ class DeviceAdamSolver:
         ctl, costs = rec.data_ptr(), rec.data_ptr() + nctl
         es = L.EarlyStop()
         es.relative_min_delta, es.patience, es.enabled = float(relative_min_delta), int(patience), int(bool(early_stopping))
+        f = fields_struct(*f2)  # (refuses tensors that are not on the device)
         st = L.stream_ptr()
         ws = workspace(dev, st)  # held until the solve has ended
         wp, wn = ws.get(g, dev)
-        f = fields_struct(*f2)
         lib = L.lib()
         if nbitmax > 0:
             rc = lib.igm_solver_solve(L.dtype_code(U.dtype), C.byref(g), C.byref(ph), C.byref(f), L.ptr(U4), L.ptr(V4),

@@ -144,3 +144,14 @@ def test_dgrad_stack_refuses_an_output_on_its_input(lib):
                                            None)
     for g, outs in ((16384, (16384,)), (16384, (32768, 32768)), (16384, (32768, 16384, 16384))):
         assert rc(g, *outs) == 2 and b"alias" in lib.igm_last_error()
+
+
+def test_cpu_tensors_are_refused_before_any_cuda_call(lib):
+    import numpy as np
+    import torch
+    from igm_b200 import kernels as K
+    from igm_b200.solver import DeviceAdamSolver
+    U, f, dz = torch.zeros(3, 8, 8), torch.zeros(8, 8), np.array([0.5, 0.5])
+    for call in (K.energy, DeviceAdamSolver().solve):
+        with pytest.raises(ValueError, match="CUDA tensor"):
+            call(U, U, f, f, f, f, 100.0, dz)
