@@ -44,7 +44,8 @@ class DeviceAdamSolver:
         g = L.make_grid(B, nz, ny, nx, dx, dzeta)
         ph = phys if isinstance(phys, L.Physics) else L.make_physics(phys)
         # the start is read where it lies (iteration 0 reads it, later ones the two working pairs)
-        U4, V4 = (t if t.is_contiguous() and t.data_ptr() % 16 == 0 else t.clone() for t in (U4, V4))
+        # unless a copy is needed for its layout, its alignment or a negation that is still to be done
+        U4, V4 = (t if t.is_contiguous() and t.data_ptr() % 16 == 0 and not t.is_neg() else t.clone() for t in (U4, V4))
         U0, V0, U1, V1, mU, mV, vU, vV = (torch.empty_like(U4) for _ in range(8))
         # control block and costs in one buffer: one copy to the host
         nctl = (C.sizeof(L.SolverCtl) + 63) // 64 * 64

@@ -191,3 +191,13 @@ def test_zero_epsilon_without_a_gradient_is_not_a_number():
     with pytest.raises(L.IgmError) as ei:
         DeviceAdamSolver(epsilon=0.0).solve(Z, Z, *f, 100.0, dz, nbitmax=5)
     assert ei.value.status == 3
+
+
+def test_lazily_negated_start():
+    """A start whose memory holds the opposite sign (a negated view) is copied."""
+    st = O.valley_glacier(40, 36, 100.0, seed=4)
+    dz = O.compute_zeta_dzeta(O.compute_levels(5, 4.0))[1].numpy()
+    f = [dev(st[k]) for k in ["thk", "usurf", "arrhenius", "slidingco"]]
+    U = torch.randn(5, 40, 36, device="cuda") * 10
+    got, ref = (DeviceAdamSolver().solve(s, s, *f, 100.0, dz, nbitmax=2) for s in (torch._neg_view(U), -U))
+    assert torch.equal(got[0], ref[0]) and torch.equal(got[1], ref[1])
