@@ -1933,8 +1933,8 @@ static int stack_launch(int batch, int height, int width, int nlayers, const voi
 // Output rows per tile of the stack.  While every tile of a layer can have an SM of its own, a layer
 // takes one tile's latency (load, MMAs, store, flag), which shrinks with the tile: the fewest rows
 // whose tiles still fit the SMs.  Above that the tiles queue, and the taller tile re-reads fewer halo
-// rows and hands over less often.  15 layers: 100 x 100 111 us with 8 rows, 62 with 2; 8 x 64 x 64 123
-// us with 8, 87 with 4; 1000 x 1000 the whole network is 4 % slower with 4 rows than with 8.
+// rows and hands over less often.  15 layers: 100 x 100 103 us with 8 rows, 66 with 2; 8 x 64 x 64 110
+// us with 8, 82 with 4; 1000 x 1000 the whole network is 4 % slower with 4 rows than with 8.
 static int stack_rows(int batch, int height, int width) {
   const long long strips = (long long)batch * ((width + kTW - 1) / kTW);
   for (int r = 2; r < kRows; r *= 2)
@@ -2067,8 +2067,8 @@ extern "C" size_t igm_conv3x3_chain_flags_len(int batch, int height, int width, 
 
 // A pass of the chain reads two halo rows above and below each piece of a run of rows and takes 8 us from
 // the last pass's flags to its own, so it pays with long runs.  16 layers, stack and first layer against
-// the chain, us: 20 rows per SM (500 x 750) 159 / 181, 27 (2 x 500 x 500) 192 / 207, 38 (700 x 1003) 255 / 251, 54
-// (1000 x 1000) 362 / 324, 235 (2048 x 2048) 1535 / 1229, 913 (4096 x 4096) 6190 / 5390.  With every activation kept it
+// the chain, us: 20 rows per SM (500 x 750) 162 / 187, 27 (2 x 500 x 500) 198 / 214, 38 (700 x 1003) 258 / 259, 54
+// (1000 x 1000) 357 / 331, 235 (2048 x 2048) 1490 / 1200, 913 (4096 x 4096) 6248 / 4733.  With every activation kept it
 // saves reads only; the whole network's forward then takes, stack / chain: 54 rows 428 / 438, 108 (8 x 500 x 500)
 // 911 / 806, 235 1915 / 1732.
 extern "C" int igm_conv3x3_chain_pays(int batch, int height, int width, int keep_all) {

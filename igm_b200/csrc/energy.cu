@@ -135,7 +135,8 @@ template <> __device__ __forceinline__ Two<float> rcbrt2<float>(Two<float> x) {
 // amplifies every rounding difference).  A zero moment steps by zero: off the
 // ice every node's gradient and moments are zero, which the square root and the
 // division would each take their slow paths for: an iteration at 1000 x 1000 x
-// 10, half of it ice, 173.5 -> 146 us, at 100 x 100 25.9 -> 22.1.
+// 10, half of it ice, 172.6 us without this and 146.5 with, in FP64 at 400 x 400
+// 85.9 and 68 (the launches then as they were; now 143 and, with the skip, 60).
 // FP32 with other copies than TMA's divides all the same (ZERO false): there ice
 // everywhere paid more for the test than bare ground gained, 701 x 1003 x 10 with
 // and without it 155 and 130 us, half ice 148 and 150; 2000 x 2001 795 and 680,
@@ -279,7 +280,7 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
   // negative), fixed at compile time so that its branches and generic powers drop out
   // Bare warps skip their layers, but not in the FP32 iteration, where the zero steps (adam_step) already save what
   // bare ground can: with the skip half ice at 1000 x 1000 x 10 is 147 us either way and all ice 163 us, without it
-  // 153.  FP64 there: half ice 290 us with it and 324 without, all ice 351 and 348.
+  // 153.  FP64 there: half ice 289 us with it and 324 without, all ice 350 and 348.
   constexpr bool kSkip = STD && (MODE != kAdamStep || sizeof(T) == 8);
   constexpr bool kZeroSteps = LOAD == kLoadTma || sizeof(T) == 8;  // adam_step
   const bool glen3 = STD || a.glen3, weert3 = STD || a.weert3, fnge = !STD && a.fnge;
@@ -1162,9 +1163,9 @@ static int field_maps(StencilMaps* maps, const igm_fields* f, const igm_grid* g)
 
 // TMA needs 16-byte aligned bases and a row pitch that is a multiple of 16 bytes; with another pitch (three
 // widths in four) the aligned bases allow 16-byte copies, a thread's one piece per array and level where
-// the elements took 2.2 copies with an address each.  701 x 1003 x 10 FP32: energy 61.5 -> 51.3 us, energy and
-// adjoint 99 -> 70; a solver iteration at 1003 x 701 x 10 202 -> 112.  (A bulk copy per box row, issued by one
-// warp: 84, 145 and 332 us.)
+// the elements took 2.2 copies with an address each.  701 x 1003 x 10 FP32, half ice: energy 58.5 -> 51.7 us, energy
+// and adjoint 97 -> 72, a solver iteration 190 -> 150.  (A bulk copy per box row, issued by one warp: 84 us, 145 and
+// more than the element copies' iteration.)
 template <typename T>
 static StencilLoad stencil_load(const igm_grid* g, std::initializer_list<const void*> ptrs) {
   for (const void* p : ptrs)

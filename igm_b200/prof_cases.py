@@ -67,7 +67,8 @@ def main():
     V = torch.as_tensor(rng.normal(0, 20, (nz, N, N)).astype(np.float32)).cuda()
     K.energy(U, V, *f, 50.0, dz)                                  # stencil: energy
     K.energy(U, V, *f, 50.0, dz, grad=True)                       # stencil: energy + adjoint
-    DeviceAdamSolver().solve(U, V, *f, 50.0, dz, nbitmax=1, early_stopping=False, mask=False)  # fused Adam step
+    DeviceAdamSolver().solve(U, V, *f, 50.0, dz, nbitmax=2, early_stopping=False, mask=False)  # fused Adam steps: the
+    # first from moments taken as zero, the second reads them
     ub, vb = U[0].contiguous(), V[0].contiguous()
     K.transport_step(ub, vb, f[0], f[1], None, 50.0, 0.01)       # transport
     topg = torch.as_tensor(st["topg"]).cuda()

@@ -135,7 +135,8 @@ IGM_API int igm_version(void);
 /* Number of kernels this library has launched in the process (all threads). */
 IGM_API long long igm_launch_count(void);
 
-/* Bytes of scratch the energy / solver / reduction calls need for this grid. */
+/* Bytes of scratch the energy / solver / reduction calls need for this grid.  Calls
+ * whose kernels may run at the same time (two streams) must not share one. */
 IGM_API size_t igm_workspace_size(const igm_grid* grid);
 
 /* ---------------------------------------------------------------------------
@@ -150,6 +151,12 @@ IGM_API size_t igm_workspace_size(const igm_grid* grid);
  *     reference's COST is (terms[0]+terms[1]+terms[2]) / (batch*(ny-1)*(nx-1)).
  *   dU, dV: NULL for the energy only; otherwise they receive
  *     grad_scale * d(sum of all densities)/d(U,V), same layout as U, V.
+ * Any nx and any element-aligned pointers are taken; what they cost differs (the
+ * results do not).  With 16-byte aligned U, V and fields, rows of a multiple of
+ * 16 bytes arrive by TMA; other rows by 16-byte copies for the default physics
+ * (exponents 3 and 3, force_negative_gravitational_energy 0; not the FP64 energy
+ * alone); else element by element, which takes 1.2 to 1.8 times as long.  The
+ * solver's calls choose in the same way.
  * ------------------------------------------------------------------------- */
 IGM_API int igm_energy(int dtype, const igm_grid* grid, const igm_physics* phys, const igm_fields* fields,
                const void* U, const void* V, void* dU, void* dV, double grad_scale, double* terms,
@@ -551,7 +558,8 @@ IGM_API size_t igm_conv3x3_stack_flags_len(int batch, int height, int width, int
  * the stream is not being captured): from g (the
  * gradient of a layer's pre-activation) outs[k] = igm_conv3x3's dgrad mode with wpacks[k]
  * and act_mask masks[k] on the previous output; the same bits.  outs may alternate
- * between two buffers, g the second of them; flags and epoch as igm_conv3x3_stack. */
+ * between two buffers, g the second of them (an output that is its layer's input is
+ * refused); flags and epoch as igm_conv3x3_stack. */
 IGM_API int igm_conv3x3_stack_dgrad(int batch, int height, int width, int nlayers, const void* g, void* const* outs,
                                     const void* const* wpacks, const void* const* masks, int* flags, int epoch,
                                     float alpha, int* err, void* stream);
