@@ -34,8 +34,9 @@ class IceflowEnergy(torch.autograd.Function):
         dx, dzeta, phys, count = ctx.args
         # the incoming gradient is read by the kernel, from memory (a lazily negated view holds -gout there): no wait
         # for the forward here
-        _, dU, dV = K.energy(U, V, thk, usurf, arrhenius, slidingco, dx, dzeta, phys, grad=True,
-                             grad_out=gout.resolve_neg().contiguous(), grad_count=count)
+        g = gout.resolve_neg() if gout.is_neg() else gout
+        _, dU, dV = K.energy(U, V, thk, usurf, arrhenius, slidingco, dx, dzeta, phys, grad=True, grad_out=g.contiguous(),
+                             grad_count=count)
         return dU, dV, None, None, None, None, None, None, None
 
 
