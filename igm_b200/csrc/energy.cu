@@ -292,6 +292,7 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
   constexpr int AL = Box<T>::AL;
   constexpr bool GRAD = MODE != kEnergyOnly;
   constexpr bool ADAM = MODE == kAdamStep;
+  constexpr bool kTwoLoops = kSkip && !ADAM;  // warps with and without ice loop over the levels apart
   constexpr bool TMA = LOAD == kLoadTma, ROWS = LOAD == kLoadRows;
   constexpr uint32_t kBoxBytes = NR * BW * sizeof(T);
   constexpr int kAhead = Ring<MODE>::ahead, kStages = Ring<MODE>::stages;
@@ -713,10 +714,13 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
       } else {
         cp_async_wait<kAhead - 1>();  // this thread's copies of level k have landed
       }
-      // level k visible to all; every thread is done with the previous iteration.  (Written out: a CTA's warps
-      // may wait here in different loops, which the instruction allows, being counted by warps, and __syncthreads
-      // does not.)
-      asm volatile("barrier.sync.aligned 0;\n" ::: "memory");
+      // level k visible to all; every thread is done with the previous iteration.  A CTA's warps may wait here in
+      // different loops, which __syncthreads does not allow and the instruction without .aligned does; in the
+      // variants with one loop it cost 2 % of an iteration.
+      if (kTwoLoops)
+        asm volatile("barrier.sync 0;\n" ::: "memory");
+      else
+        __syncthreads();
       issue_next();
       if (GRAD && !FIRST && k >= 2) finish(k - 2, st_m2);
 
@@ -874,14 +878,14 @@ __global__ void __launch_bounds__(kCW* TYP, MinBlocks<T, MODE>::value)
         cons_ph ^= 1u;
       }
     };
-    // Energy and adjoint: warps with ice run a loop of their own, without the test (the barriers count warps,
-    // whichever loop they are in).  With one loop for both, ice everywhere, 1000 x 1000 x 10: the adjoint 103 us,
+    // Energy and adjoint: warps with ice run a loop of their own, without the test (the barrier in it takes warps from
+    // both).  With one loop for both, ice everywhere, 1000 x 1000 x 10: the adjoint 103 us,
     // now 98.2, the energy 55.8 and 53.7.  The FP64 iteration keeps one (two: half ice 291 us, all ice 355; one:
     // 290 and 351).
     using InLoop = std::integral_constant<int, kSkip && ADAM ? 2 : 0>;
-    using Bare = std::integral_constant<int, kSkip && !ADAM ? 1 : 0>;
+    using Bare = std::integral_constant<int, kTwoLoops ? 1 : 0>;
     constexpr int kBareUnroll = GRAD ? 1 : 2;  // unrolled by two, the adjoint with ice everywhere takes 99.0 us
-    if (Bare::value && bare) {
+    if (kTwoLoops && bare) {
       level(0, std::true_type{}, Bare{});
 #pragma unroll kBareUnroll
       for (int k = 1; k < nz; ++k) level(k, std::false_type{}, Bare{});
